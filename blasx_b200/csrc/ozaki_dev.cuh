@@ -995,7 +995,6 @@ struct Parts {
     int *ea, *fb;
     int8_t *Y, *X;
     uint8_t *U;
-    size_t stats_bytes;  // sa and sb, contiguous from sa.amax: cleared before the statistics
 };
 inline Parts carve_parts(const Gemm &g, const Plan &pl, void *ws) {
     const int64_t L = kMaxModuli;
@@ -1003,14 +1002,16 @@ inline Parts carve_parts(const Gemm &g, const Plan &pl, void *ws) {
     Parts p;
     p.err = cv.take<int>(1);
     p.dec = cv.take<Decision>(1);
-    p.sa = RowStats{cv.take<double>(pl.M), cv.take<double>(pl.M), cv.take<double>(pl.M), cv.take<int>(pl.M)};
-    p.sb = RowStats{cv.take<double>(pl.N), cv.take<double>(pl.N), cv.take<double>(pl.N), cv.take<int>(pl.N)};
+    // the flags (arrival counters of the standalone statistics) directly
+    // after the decision: one range to clear
+    int *fa = cv.take<int>(pl.M), *fb = cv.take<int>(pl.N);
+    p.sa = RowStats{cv.take<double>(pl.M), cv.take<double>(pl.M), cv.take<double>(pl.M), fa};
+    p.sb = RowStats{cv.take<double>(pl.N), cv.take<double>(pl.N), cv.take<double>(pl.N), fb};
     p.ea = cv.take<int>(pl.M);
     p.fb = cv.take<int>(pl.N);
     p.Y = cv.take<int8_t>(size_t(L) * pl.Ip * pl.Kp);
     p.X = pl.alias ? p.Y : cv.take<int8_t>(size_t(L) * pl.Jx * pl.Kp);
     p.U = cv.take<uint8_t>(size_t(L) * pl.Jx * pl.Ip);
-    p.stats_bytes = size_t(reinterpret_cast<char *>(p.ea) - reinterpret_cast<char *>(p.sa.amax));
     return p;
 }
 
