@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(kThreads, 1) executor_kernel(const ExecArgs a)
     pipe.done = oz::su32(s_bars + 2 * oz::kStages + 4);
     pipe.tmem_slot = &s_tmem_slot;
     pipe.abort_flag = &s_abort;
-    if (tid == 0) oz::residue_pipe_init(pipe);
+    if (tid == 0) oz::residue_pipe_init<1>(pipe);
     if (warp == 1) oz::tmem_alloc_all(pipe.tmem_slot);
     oz::tc_fence_before();
     __syncthreads();
@@ -413,7 +413,8 @@ __global__ void __launch_bounds__(kThreads, 1) executor_kernel(const ExecArgs a)
             case kResidue: {
                 const int nmod = __ldcg(&d.dec->nmod);
                 if (nmod > 0) {
-                    const oz::TileCoord c = oz::decode(t.first, int(d.res_tiles_j), int(d.res_tiles_i), 0);
+                    const oz::TileCoord c = oz::decode(uint32_t(t.first), uint32_t(d.res_tiles_j),
+                                                       uint32_t(d.res_tiles_i), 16u, 0);
                     oz::TileSeq q;
                     q.raster = false;
                     q.first = q.step = q.end = 0;
@@ -429,7 +430,7 @@ __global__ void __launch_bounds__(kThreads, 1) executor_kernel(const ExecArgs a)
                         asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(my) : "memory");
                         asm volatile("fence.proxy.async.global;" ::: "memory");
                     }
-                    oz::residue_roles(mx, my, ta, q, nmod, pipe, tmem, pos, warp, lane, t.stall != 0);
+                    oz::residue_roles<1>(mx, my, ta, q, nmod, pipe, tmem, pos, warp, lane, t.stall != 0);
                 }
                 break;
             }
@@ -463,7 +464,7 @@ __global__ void __launch_bounds__(kThreads, 1) executor_kernel(const ExecArgs a)
             // a residue pipeline gave up; its copies and MMAs have drained, so
             // its barriers can be initialised again
             __syncthreads();
-            if (tid == 0) oz::residue_pipe_init(pipe);
+            if (tid == 0) oz::residue_pipe_init<1>(pipe);
             pos = oz::RolePos{};
             __syncthreads();
         }

@@ -20,10 +20,11 @@ namespace {
 
 __global__ void __launch_bounds__(kThreadsTC, 1)
     residue_gemm_kernel(const __grid_constant__ CUtensorMap mapX,
-                        const __grid_constant__ CUtensorMap mapY, const TcArgs a) {
+                        const __grid_constant__ CUtensorMap mapY, const TcArgs a,
+                        const uint32_t gj) {
     const int nmod = a.dec->nmod;
-    const int tiles_j = a.tjn, tiles_i = int(a.Ip / kTileI);
-    const int64_t total = int64_t(nmod) * tiles_j * tiles_i;
+    const uint32_t tiles_j = uint32_t(a.tjn), tiles_i = uint32_t(a.Ip / kTileI);
+    const uint32_t total = uint32_t(nmod) * tiles_j * tiles_i;  // fits: checked by the launch
     if (total == 0) return;  // native fallback chosen on the device
 
     extern __shared__ uint8_t smem_raw[];
@@ -31,7 +32,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const ResiduePipe p = residue_pipe_at(smem);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (threadIdx.x == 0) residue_pipe_init(p);
+    if (threadIdx.x == 0) residue_pipe_init<2>(p);
     if (warp == 1) tmem_alloc_all(p.tmem_slot);
     tc_fence_before();
     __syncthreads();
@@ -46,10 +47,11 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
     q.end = total;
     q.tiles_j = tiles_j;
     q.tiles_i = tiles_i;
+    q.gj = gj;
     q.tj0 = a.tj0;
     q.tj = q.ti = 0;
     RolePos pos;
-    residue_roles(&mapX, &mapY, a, q, seq_count(q, nmod), p, tmem, pos, warp, lane,
+    residue_roles<2>(&mapX, &mapY, a, q, seq_count(q, nmod), p, tmem, pos, warp, lane,
                   int(blockIdx.x) == a.stall_cta);
     tc_fence_before();
     __syncthreads();
@@ -120,10 +122,15 @@ int launch_residue_gemm(const int8_t *X, const int8_t *Y, uint8_t *U, int64_t Jp
     take_stall(&a.wait_cycles, &a.stall_cta);
     const int64_t tiles_upper = int64_t(kMaxModuli) * tj_count * (Ip / kTileI);
     if (tiles_upper == 0) return BLASX_OK;
+    if (tiles_upper > INT32_MAX) return set_error(BLASX_ERR_UNSUPPORTED, "residue GEMM: too many tiles");
     int64_t grid = tiles_upper < num_sms ? tiles_upper : num_sms;
     if (max_cta_tiles > 0) grid = std::max<int64_t>(grid, (tiles_upper + max_cta_tiles - 1) / max_cta_tiles);
     grid = std::min<int64_t>(grid, INT32_MAX);
-    residue_gemm_kernel<<<unsigned(grid), kThreadsTC, kSmemBytes, s>>>(mx, my, a);
+    // j-tiles per raster group: a group's X panel is read again for every
+    // i-tile. 32 tiles of up to 8192 k (32 MB) stay in L2 meanwhile; longer
+    // panels do not, and 16 keep the operands of one wave of tiles smallest.
+    const uint32_t gj = Kp > 8192 ? 16u : 32u;
+    residue_gemm_kernel<<<unsigned(grid), kThreadsTC, kSmemBytes, s>>>(mx, my, a, gj);
     BX_CUDA(cudaGetLastError());
     count_launch();
     return BLASX_OK;

@@ -17,7 +17,8 @@
 //               tcgen05.commit frees the stage; two 256-column accumulators
 //               let the epilogue of one tile overlap the MMAs of the next;
 //   warps 2..5  epilogue: tcgen05.ld 32x32b.x32, INT32 -> residue mod m_l,
-//               16-byte stores of uint8.
+//               16-byte stores of uint8 (with GROUPS = 2, warps 2..9, each
+//               group of four taking half of a tile's columns).
 // Every mbarrier wait is bounded (a limit in clock cycles, about one second
 // by default); on expiry the CTA raises a device error word and an abort flag
 // in shared memory, the producer waits (bounded) for its copies in flight,
@@ -42,12 +43,16 @@ constexpr int kStages = 4;
 constexpr int kXBytes = kTileJ * kTileK;  // 16 KB
 constexpr int kYBytes = kTileI * kTileK;  // 32 KB
 constexpr int kStageBytes = kXBytes + kYBytes;
-constexpr int kThreadsTC = 192;
+constexpr int kThreadsTC = 320;  // the standalone kernel: two epilogue groups
 constexpr uint32_t kTmemCols = 512;
 constexpr int kAccCols = 256;
 constexpr long long kWaitCycles = 2000000000LL;  // default wait limit: ~1 s at 1.9 GHz
 
-static __constant__ int c_mod[kMaxModuli];
+// Per modulus m, the constants of residue_of (below).
+struct ModRow {
+    uint32_t m, w, cb, magic;
+};
+static __constant__ ModRow c_mod[kMaxModuli];
 
 struct TcArgs {
     int64_t Jp, Ip, Kp;
@@ -75,10 +80,13 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+// The hint lets a waiting warp sleep up to 20 us instead of polling: twelve
+// polling warps cost power that the tensor cores can use (2% at 4096 x 4096 x
+// 1024).
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
-        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 20000;\n"
         "selp.u32 %0, 1, 0, p;\n}"
         : "=r"(ok)
         : "r"(bar), "r"(parity)
@@ -91,7 +99,7 @@ __device__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_fla
     const long long t0 = clock64();
     for (uint32_t it = 0;; ++it) {
         if (mbar_try(bar, parity)) return true;
-        if ((it & 63) == 63) {
+        if ((it & 15) == 15) {
             if (abort_flag && *abort_flag) return false;
             if (clock64() - t0 > limit) return false;
         }
@@ -158,32 +166,54 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// x mod m in [0, m) for |x| < 2^31, m <= 256: a float quotient estimate is off
-// by at most one (|x| * 2^-24 / m < 1), corrected by two compares.
-__device__ __forceinline__ uint32_t mod_small(int32_t x, int32_t m, float inv_m) {
-    const int32_t q = __float2int_rd(__int2float_rn(x) * inv_m);
-    int32_t r = x - q * m;
-    r += (r < 0) ? m : 0;
-    r -= (r >= m) ? m : 0;
-    return uint32_t(r);
+// x mod m in [0, m) for any int32 x: the bytes b_k of x + 2^31 give
+//   s = sum_k b_k (2^(8k) mod m) + (-2^31 mod m) <= 4 * 255 * 255 + 255 < 2^20,
+// one byte dot product (DP4A), congruent to x; floor(s / m) is the high word
+// of s * ceil(2^32 / m), exact for s < 2^20 and m <= 256. Four integer
+// instructions and no conversion: the float quotient with two corrections
+// that it replaced spent two conversions (a quarter-rate pipe) and eight
+// other instructions, and with four epilogue warps a tile's epilogue took
+// longer than its MMAs below K = 2500. With this form and eight warps whole
+// calls fell from 265 to 248 us (FP64 2048^3), from 525 to 497 (complex128
+// 2401 x 1639 x 1203), from 154 to 145 (FP32 3001 x 1777 x 999) and from 350
+// to 321 (DSYRK 4000 x 1000).
+__device__ __forceinline__ uint32_t residue_of(uint32_t x, const ModRow &c) {
+    const uint32_t s = __dp4a(x ^ 0x80000000u, c.w, c.cb);
+    return s - __umulhi(s, c.magic) * c.m;
+}
+
+// 32 accumulators reduced mod m and stored as 32 consecutive bytes (32-byte
+// aligned: one whole sector per store).
+__device__ __forceinline__ void store_residues32(uint8_t *out, const uint32_t (&r)[32], const ModRow &c) {
+    uint32_t w[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const uint32_t a = residue_of(r[4 * q], c), b = residue_of(r[4 * q + 1], c);
+        const uint32_t d = residue_of(r[4 * q + 2], c), e = residue_of(r[4 * q + 3], c);
+        w[q] = __byte_perm(__byte_perm(a, b, 0x0040u), __byte_perm(d, e, 0x0040u), 0x5410u);
+    }
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(out), "r"(w[0]), "r"(w[1]), "r"(w[2]),
+                 "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                 : "memory");
 }
 
 struct TileCoord {
     int l, tj, ti;
 };
-__device__ __forceinline__ TileCoord decode(int64_t tile, int tiles_j, int tiles_i, int tj0) {
-    constexpr int GJ = 16;  // j-tiles per raster group (operand panels stay in L2)
-    const int64_t per_mod = int64_t(tiles_j) * tiles_i;
+// Tile t of the raster order over (modulus, j-tile, i-tile): groups of gj
+// j-tiles, inside a group one i-tile after the other (32-bit: the 64-bit
+// divisions took hundreds of cycles of every role at each tile).
+__device__ __forceinline__ TileCoord decode(uint32_t t, uint32_t tiles_j, uint32_t tiles_i, uint32_t gj, int tj0) {
+    const uint32_t per_mod = tiles_j * tiles_i;
     TileCoord c;
-    c.l = int(tile / per_mod);
-    const int64_t t = tile % per_mod;
-    const int64_t per_group = int64_t(GJ) * tiles_i;
-    const int group = int(t / per_group);
-    const int first = group * GJ;
-    const int gsize = min(GJ, tiles_j - first);
-    const int64_t in = t % per_group;
-    c.tj = tj0 + first + int(in % gsize);
-    c.ti = int(in / gsize);
+    c.l = int(t / per_mod);
+    t -= uint32_t(c.l) * per_mod;
+    const uint32_t group = t / (gj * tiles_i), first = group * gj;
+    t -= first * tiles_i;
+    const uint32_t gsize = min(gj, tiles_j - first);
+    const uint32_t row = t / gsize;
+    c.tj = tj0 + int(first + t - row * gsize);
+    c.ti = int(row);
     return c;
 }
 
@@ -227,14 +257,14 @@ __device__ __forceinline__ ResiduePipe residue_pipe_at(uint8_t *base) {
 
 // Initialises the barriers and clears the abort flag (one thread; a CTA
 // barrier must follow before any role uses them).
-__device__ __forceinline__ void residue_pipe_init(const ResiduePipe &p) {
+template <int GROUPS> __device__ __forceinline__ void residue_pipe_init(const ResiduePipe &p) {
     for (int s = 0; s < kStages; ++s) {
         mbar_init(p.full0 + 8 * s, 1);
         mbar_init(p.empty0 + 8 * s, 1);
     }
     for (int b = 0; b < 2; ++b) {
         mbar_init(p.tfull0 + 8 * b, 1);
-        mbar_init(p.tempty0 + 8 * b, 4);
+        mbar_init(p.tempty0 + 8 * b, 4 * GROUPS);
     }
     mbar_init(p.done, 1);
     *p.abort_flag = 0;
@@ -266,28 +296,30 @@ struct RolePos {
 // moduli 0 .. nmod-1 of one C tile (tj, ti).
 struct TileSeq {
     bool raster;
-    int64_t first, step, end;   // raster walk
-    int tiles_j, tiles_i, tj0;  // raster geometry
-    int tj, ti;                 // one C tile
+    uint32_t first, step, end;             // raster walk
+    uint32_t tiles_j, tiles_i, gj;         // raster geometry
+    int tj0;
+    int tj, ti;                            // one C tile
 };
-__device__ __forceinline__ TileCoord seq_tile(const TileSeq &q, int64_t s) {
-    if (q.raster) return decode(q.first + s * q.step, q.tiles_j, q.tiles_i, q.tj0);
+__device__ __forceinline__ TileCoord seq_tile(const TileSeq &q, uint32_t s) {
+    if (q.raster) return decode(q.first + s * q.step, q.tiles_j, q.tiles_i, q.gj, q.tj0);
     return TileCoord{int(s), q.tj, q.ti};
 }
-__device__ __forceinline__ int64_t seq_count(const TileSeq &q, int nmod) {
+__device__ __forceinline__ uint32_t seq_count(const TileSeq &q, int nmod) {
     if (q.raster) return q.end > q.first ? (q.end - q.first + q.step - 1) / q.step : 0;
-    return nmod;
+    return uint32_t(nmod);
 }
 
 // The three roles of the pipeline over the tiles of q, for the calling thread
-// (warp 0 lane 0: TMA producer; warp 1 lane 0: MMA issuer; warps 2..5:
-// epilogue; every other thread returns at once). On a wait that runs out the
+// (warp 0 lane 0: TMA producer; warp 1 lane 0: MMA issuer; warps 2 to
+// 1 + 4 GROUPS: epilogue; every other thread returns at once). On a wait that runs out the
 // CTA's abort flag and the device error word are raised, the producer waits
 // (bounded) for its copies in flight and the MMA issuer for its MMAs; the
 // pipeline must then be initialised again before further use. mapX / mapY:
 // generic addresses of the tensor maps (kernel parameters or global memory).
+template <int GROUPS>
 __device__ __forceinline__ void residue_roles(const CUtensorMap *mapX, const CUtensorMap *mapY,
-                                              const TcArgs &a, const TileSeq &q, int64_t count,
+                                              const TcArgs &a, const TileSeq &q, uint32_t count,
                                               const ResiduePipe &p, uint32_t tmem, RolePos &pos,
                                               int warp, int lane, bool stall) {
     const int num_kb = int(a.Kp / kTileK);
@@ -300,7 +332,7 @@ __device__ __forceinline__ void residue_roles(const CUtensorMap *mapX, const CUt
             // test hook: a stalled pipeline issues nothing for its second stage,
             // so that the MMA issuer's wait for that stage runs out
             int skip = stall ? 1 : -1;
-            for (int64_t t = 0; t < count && ok; ++t) {
+            for (uint32_t t = 0; t < count && ok; ++t) {
                 const TileCoord c = seq_tile(q, t);
                 if (!tile_needed(c, a)) continue;
                 for (int kb = 0; kb < num_kb; ++kb) {
@@ -337,7 +369,7 @@ __device__ __forceinline__ void residue_roles(const CUtensorMap *mapX, const CUt
             // ---------------- MMA issuer ----------------
             constexpr uint32_t idesc = idesc_i8(kTileJ, kTileI);
             bool ok = true;
-            for (int64_t t = 0; t < count && ok; ++t) {
+            for (uint32_t t = 0; t < count && ok; ++t) {
                 if (!tile_needed(seq_tile(q, t), a)) continue;
                 if (!mbar_wait(p.tempty0 + 8 * pos.acc, pos.acc_phase ^ 1, abort_flag, a.wait_cycles)) {
                     ok = false;
@@ -372,14 +404,15 @@ __device__ __forceinline__ void residue_roles(const CUtensorMap *mapX, const CUt
             mbar_wait(p.done, pos.done_phase, nullptr, a.wait_cycles);
             pos.done_phase ^= 1;
         }
-    } else if (warp < 6) {
-        // ---------------- epilogue (warps 2..5) ----------------
+    } else if (warp < 2 + 4 * GROUPS) {
+        // ---------------- epilogue ----------------
         const int quarter = warp & 3;  // TMEM lanes 32*quarter .. +31
-        for (int64_t t = 0; t < count; ++t) {
+        constexpr int COLS = kTileI / GROUPS;
+        const int col0 = (warp - 2) / 4 * COLS;
+        for (uint32_t t = 0; t < count; ++t) {
             const TileCoord c = seq_tile(q, t);
             if (!tile_needed(c, a)) continue;
-            const int32_t m = c_mod[c.l];
-            const float inv_m = 1.0f / float(m);
+            const ModRow mod = c_mod[c.l];
             if (!mbar_wait(p.tfull0 + 8 * pos.acc, pos.acc_phase, abort_flag, a.wait_cycles)) {
                 if (lane == 0) atomicOr(a.err, 4);
                 *abort_flag = 1;
@@ -387,23 +420,13 @@ __device__ __forceinline__ void residue_roles(const CUtensorMap *mapX, const CUt
             }
             tc_fence_after();
             const int64_t j = int64_t(c.tj) * kTileJ + quarter * 32 + lane;
-            uint8_t *out = a.U + int64_t(c.l) * a.Jp * a.Ip + j * a.Ip + int64_t(c.ti) * kTileI;
-            const uint32_t tbase = tmem + (uint32_t(quarter * 32) << 16) + uint32_t(pos.acc * kAccCols);
+            uint8_t *out = a.U + int64_t(c.l) * a.Jp * a.Ip + j * a.Ip + int64_t(c.ti) * kTileI + col0;
+            const uint32_t tbase = tmem + (uint32_t(quarter * 32) << 16) + uint32_t(pos.acc * kAccCols + col0);
 #pragma unroll 1
-            for (int ch = 0; ch < kTileI / 32; ++ch) {
+            for (int ch = 0; ch < COLS / 32; ++ch) {
                 uint32_t r[32];
                 tmem_ld32(tbase + uint32_t(ch * 32), r);
-                uint32_t w[8];
-#pragma unroll
-                for (int qq = 0; qq < 8; ++qq) {
-                    w[qq] = mod_small(int32_t(r[4 * qq]), m, inv_m) |
-                            (mod_small(int32_t(r[4 * qq + 1]), m, inv_m) << 8) |
-                            (mod_small(int32_t(r[4 * qq + 2]), m, inv_m) << 16) |
-                            (mod_small(int32_t(r[4 * qq + 3]), m, inv_m) << 24);
-                }
-                uint4 *o = reinterpret_cast<uint4 *>(out + ch * 32);
-                o[0] = make_uint4(w[0], w[1], w[2], w[3]);
-                o[1] = make_uint4(w[4], w[5], w[6], w[7]);
+                store_residues32(out + ch * 32, r, mod);
             }
             tc_fence_before();
             __syncwarp();
@@ -446,7 +469,16 @@ int make_map(CUtensorMap *map, const void *base, int64_t rows, int64_t kp, int b
 
 // Uploads the moduli to this translation unit's constant memory on the
 // current device.
-inline cudaError_t upload_moduli() { return cudaMemcpyToSymbol(c_mod, kModuli, sizeof(kModuli)); }
+inline cudaError_t upload_moduli() {
+    ModRow rows[kMaxModuli];
+    for (int l = 0; l < kMaxModuli; ++l) {
+        const uint32_t m = uint32_t(kModuli[l]);
+        const auto pw = [m](int bits) { return uint32_t((uint64_t(1) << bits) % m); };
+        rows[l] = ModRow{m, pw(0) | pw(8) << 8 | pw(16) << 16 | pw(24) << 24, (m - pw(31)) % m,
+                         uint32_t(((uint64_t(1) << 32) + m - 1) / m)};
+    }
+    return cudaMemcpyToSymbol(c_mod, rows, sizeof rows);
+}
 
 }  // namespace
 }  // namespace oz
