@@ -3,11 +3,11 @@
 // (kernels_dmma.cu) and the serving executor (executor.cu).
 //
 // One CTA of Tile<CPLX, G>::THREADS threads computes one C tile:
-//   * 8 warps in a 2 x 4 grid (FP64 128x128 tile, complex128 64x128), or 4
-//     warps in a 2 x 2 grid (FP64 64x64 tile, G = 1); a warp owns a block of
-//     accumulators in registers;
-//   * operand tiles are staged global -> shared through a 3-stage cp.async
-//     ring. Each operand keeps the contiguity it has in global memory: a
+//   * 8 warps in a 2 x 4 grid (128x128, complex128 64x128 tiles), or 4 warps
+//     in a 2 x 2 grid (smaller tiles); a warp owns a block of accumulators in
+//     registers;
+//   * operand tiles are staged global -> shared through a 3- or 4-stage
+//     cp.async ring. Each operand keeps the contiguity it has in global memory: a
 //     k-contiguous source (A transposed, B not) lands as [m][k] rows padded
 //     by 4 doubles, an m/n-contiguous source as [k][m] rows padded by 4, so
 //     every copy is a 16-byte cp.async along the contiguous direction and
@@ -29,22 +29,49 @@
 namespace bx {
 namespace dev {
 
-// CTA geometry. G selects the FP64 variant: 0 = a 128x128 C tile, 8 warps
-// (2 x 4) of 64x32 accumulators each; 1 = a 64x64 C tile, 4 warps (2 x 2) of
-// 32x32, two CTAs per SM, for problems with too few 128x128 tiles to occupy
-// every SM (one CTA computes its whole K extent, at one SM's FP64 rate).
+// CTA geometry G (the launch chooses, kernels_dmma.cu). All FP64 tiles run
+// mma.m16n8k16; what differs is how many warps share a scheduler and how
+// finely a problem is cut. Measured on a full GPU (8192 x 8192 x 2048, FP64
+// pipe 37.1 TF/s) and, with two 64x64 tiles per SM, at 1024^3:
+//   0  128x128 (complex128 64x128), 8 warps, 1 CTA per SM: 30.8 TF/s; the
+//      serving executor's tile (its CTAs have 8 warps);
+//   1  64x64, 4 warps, BK 16 in 4 stages, 3 CTAs per SM: 32.4 TF/s (BK 32 in 3
+//      stages, 2 CTAs: 30.8); complex128 2 CTAs per SM: 31.9;
+//   2  32x32, 4 warps, 4 CTAs per SM: 28.7 TF/s (complex128 30.8), but 512^3
+//      in 16.6 us against 33 with 64x64 tiles;
+//   3  64x48, 4 warps, 4 CTAs per SM: 31.5 TF/s; a second edge for grids that
+//      64x64 tiles leave uneven (1003 x 777 x 641: 47.7 us against 59.7).
+// Double-buffering the fragments in registers by hand was slower everywhere
+// (28.7 TF/s with tile 1): it spills where the compiler's own schedule fits.
+// The k extent of a tile can be cut over the CTAs of a cluster (SPLIT).
 template <bool CPLX, int G = 0> struct Tile;
 template <> struct Tile<false, 0> {
-    static constexpr int THREADS = 256, WARPS_N = 4;
+    static constexpr int THREADS = 256, WARPS_N = 4, PER_SM = 1;
     static constexpr int BM = 128, BN = 128, MT = 4, NT = 4, BK = 32, STAGES = 3;
 };
 template <> struct Tile<false, 1> {
-    static constexpr int THREADS = 128, WARPS_N = 2;
-    static constexpr int BM = 64, BN = 64, MT = 2, NT = 4, BK = 32, STAGES = 3;
+    static constexpr int THREADS = 128, WARPS_N = 2, PER_SM = 3;
+    static constexpr int BM = 64, BN = 64, MT = 2, NT = 4, BK = 16, STAGES = 4;
+};
+template <> struct Tile<false, 2> {
+    static constexpr int THREADS = 128, WARPS_N = 2, PER_SM = 4;
+    static constexpr int BM = 32, BN = 32, MT = 1, NT = 2, BK = 32, STAGES = 3;
+};
+template <> struct Tile<false, 3> {
+    static constexpr int THREADS = 128, WARPS_N = 2, PER_SM = 4;
+    static constexpr int BM = 64, BN = 48, MT = 2, NT = 3, BK = 16, STAGES = 3;
 };
 template <> struct Tile<true, 0> {
-    static constexpr int THREADS = 256, WARPS_N = 4;
+    static constexpr int THREADS = 256, WARPS_N = 4, PER_SM = 1;
     static constexpr int BM = 64, BN = 128, MT = 2, NT = 4, BK = 16, STAGES = 3;
+};
+template <> struct Tile<true, 1> {
+    static constexpr int THREADS = 128, WARPS_N = 2, PER_SM = 2;
+    static constexpr int BM = 64, BN = 64, MT = 2, NT = 4, BK = 16, STAGES = 3;
+};
+template <> struct Tile<true, 2> {
+    static constexpr int THREADS = 128, WARPS_N = 2, PER_SM = 4;
+    static constexpr int BM = 32, BN = 32, MT = 1, NT = 2, BK = 16, STAGES = 3;
 };
 
 // Shared-memory geometry of one operand tile (rows x k) for a given source
@@ -72,6 +99,7 @@ struct DmmaParams {
     int tiles_m, tiles_n;
     int vec_a, vec_b;  // 16-byte copies allowed (ld even, base 16-byte aligned)
     const int *guard;  // when set, run only if *guard == 0
+    int *queue;        // tile counter of a guarded launch (Gemm::queue)
     int uplo;          // triangular output: 0 all, 1 row - col <= diag, 2 row - col >= diag
     int64_t diag;
 };
@@ -169,9 +197,46 @@ __device__ __forceinline__ void load_tile(uint32_t sbase, const double *src, int
     }
 }
 
-// One C tile of one problem (`tile` in the grouped raster order below).
-template <bool CPLX, bool AKC, bool BKC, int KI, int G = 0>
-__device__ __forceinline__ void dmma_tile(const DmmaParams &p, const int tile, double *smem) {
+__device__ __forceinline__ void dmma_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// A double of the shared memory of CTA `rank` of the cluster, at the place
+// that `local` has in this CTA's.
+__device__ __forceinline__ double cluster_read(const double *local, uint32_t rank) {
+    uint32_t addr;
+    double v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(smem_u32(local)), "r"(rank));
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(addr) : "memory");
+    return v;
+}
+
+// One entry of C = alpha x + beta C.
+template <bool CPLX>
+__device__ __forceinline__ void dmma_put(const DmmaParams &p, double *cp, double xr, double xi) {
+    if (!CPLX) {
+        double v = p.alpha_re * xr;
+        if (!p.beta_zero) v = fma(p.beta_re, *cp, v);
+        *cp = v;
+    } else {
+        double vr = p.alpha_re * xr - p.alpha_im * xi;
+        double vi = p.alpha_re * xi + p.alpha_im * xr;
+        if (!p.beta_zero) {
+            const double cr = cp[0], ci = cp[1];
+            vr += p.beta_re * cr - p.beta_im * ci;
+            vi += p.beta_re * ci + p.beta_im * cr;
+        }
+        cp[0] = vr;
+        cp[1] = vi;
+    }
+}
+
+// One C tile of one problem (`tile` in the grouped raster order below). With
+// SPLIT, CTA `rank` of a cluster of `splits` takes its share of the k-tiles;
+// the partial tiles are then added in rank order through distributed shared
+// memory, each CTA finishing an equal share of the entries.
+template <bool CPLX, bool AKC, bool BKC, int KI, int G = 0, bool SPLIT = false>
+__device__ __forceinline__ void dmma_tile(const DmmaParams &p, const int tile, double *smem, int rank = 0,
+                                          int splits = 1) {
     using TL = Tile<CPLX, G>;
     constexpr int T = TL::THREADS;
     constexpr int BM = TL::BM, BN = TL::BN, MT = TL::MT, NT = TL::NT, BK = TL::BK;
@@ -196,7 +261,7 @@ __device__ __forceinline__ void dmma_tile(const DmmaParams &p, const int tile, d
     const int m0 = tm * BM, n0 = tn * BN;
     // triangular output: a tile with no entry inside computes nothing (uniform per CTA)
     if (p.uplo == 1 && int64_t(m0) - (n0 + BN - 1) > p.diag) return;
-    if (p.uplo == 2 && int64_t(m0 + BM - 1) - n0 < p.diag) return;
+    if (p.uplo == 2 && int64_t(m0 + BM - 1) - n0 < p.diag) return;  // (uniform per cluster too)
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int wm = warp / TL::WARPS_N, wn = warp % TL::WARPS_N;
@@ -226,10 +291,12 @@ __device__ __forceinline__ void dmma_tile(const DmmaParams &p, const int tile, d
 #pragma unroll
                 for (int r = 0; r < 4; ++r) acc[pl][i][j][r] = 0.0;
 
-    const int ktiles = (p.K + BK - 1) / BK;
+    const int ktiles_all = (p.K + BK - 1) / BK;
+    const int kt0 = SPLIT ? int(int64_t(ktiles_all) * rank / splits) : 0;
+    const int ktiles = SPLIT ? int(int64_t(ktiles_all) * (rank + 1) / splits) - kt0 : ktiles_all;
 #pragma unroll
     for (int s = 0; s < STAGES - 1; ++s) {
-        if (s < ktiles) load_stage(s, s);
+        if (s < ktiles) load_stage(s, kt0 + s);
         cp_async_commit();
     }
 
@@ -243,7 +310,7 @@ __device__ __forceinline__ void dmma_tile(const DmmaParams &p, const int tile, d
         __syncthreads();
         {
             const int nk = kt + STAGES - 1;
-            if (nk < ktiles) load_stage(nk % STAGES, nk);
+            if (nk < ktiles) load_stage(nk % STAGES, kt0 + nk);
             cp_async_commit();
         }
         const double *a_s = sA + (kt % STAGES) * A_STAGE;
@@ -297,6 +364,39 @@ __device__ __forceinline__ void dmma_tile(const DmmaParams &p, const int tile, d
         }
     }
     cp_async_wait<0>();
+
+    if constexpr (SPLIT) {
+        // the partial tile, by columns, in place of the operand stages
+        __syncthreads();
+        constexpr int LD = BM + 2;
+        static_assert(PLANES * BN * LD <= STAGES * (A_STAGE + B_STAGE), "the partial tile fits the stages");
+#pragma unroll
+        for (int pl = 0; pl < PLANES; ++pl)
+#pragma unroll
+            for (int i = 0; i < MT; ++i)
+#pragma unroll
+                for (int j = 0; j < NT; ++j)
+#pragma unroll
+                    for (int r = 0; r < 4; ++r)
+                        smem[(pl * BN + wn * (NT * 8) + j * 8 + 2 * t + (r & 1)) * LD + wm * (MT * 16) + i * 16 + g +
+                             (r >= 2 ? 8 : 0)] = acc[pl][i][j][r];
+        dmma_cluster_sync();
+        const int per = (BN + splits - 1) / splits;  // columns this CTA finishes
+        const int c0 = rank * per, cn = min(per, BN - c0);
+        for (int e = tid; e < cn * BM; e += T) {
+            const int r = e % BM, c = c0 + e / BM;
+            const int row = m0 + r, col = n0 + c;
+            if (row >= p.M || col >= p.N || !tri_keep(p.uplo, p.diag, row, col)) continue;
+            double x[2] = {0.0, 0.0};
+            for (int s = 0; s < splits; ++s)
+#pragma unroll
+                for (int pl = 0; pl < PLANES; ++pl)
+                    x[pl] += cluster_read(smem + (pl * BN + c) * LD + r, uint32_t(s));
+            dmma_put<CPLX>(p, p.C + (row + int64_t(col) * p.ldc) * (CPLX ? 2 : 1), x[0], x[1]);
+        }
+        dmma_cluster_sync();  // no CTA leaves while another still reads its partial tile
+        return;
+    }
 
     // epilogue: C = alpha acc + beta C (C unread when beta == 0). The C values
     // of one row block (NT x 4 per thread) are all loaded before any store of
@@ -370,6 +470,7 @@ template <bool CPLX, int G = 0> DmmaParams make_params(const Gemm &g) {
     p.vec_a = (g.lda % 2 == 0) && (reinterpret_cast<uintptr_t>(g.A) % 16 == 0);
     p.vec_b = (g.ldb % 2 == 0) && (reinterpret_cast<uintptr_t>(g.B) % 16 == 0);
     p.guard = g.guard;
+    p.queue = g.queue;
     p.uplo = g.uplo;
     p.diag = g.diag;
     return p;

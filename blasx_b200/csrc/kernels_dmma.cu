@@ -7,8 +7,9 @@
 //
 // The tile itself (DMMA fragments, the cp.async ring, the alpha / beta
 // epilogue) is dmma_tile.cuh, shared with the serving executor; this file
-// holds the launches: one CTA per C tile, with the CTA geometry chosen by
-// the estimated SM utilisation.
+// holds the launches, with the CTA geometry and the k split chosen by an
+// estimate of the time.
+#include <algorithm>
 #include <cstdint>
 #include <cstdlib>
 
@@ -21,31 +22,91 @@ namespace {
 
 using namespace dev;
 
+// One CTA per tile; or, for the emulated path's fallback, one resident set of
+// CTAs that take tiles from a counter: it usually has nothing to do, and the
+// exits of a CTA per tile took 6 us at 2048^3. (Tiles dealt out in advance
+// instead took 6% longer when 4096 x 3000 x 2500 did fall back.)
 template <bool CPLX, bool AKC, bool BKC, int KI, int G>
-__global__ void __launch_bounds__(Tile<CPLX, G>::THREADS, 1) dmma_gemm_kernel(const DmmaParams p) {
+__global__ void __launch_bounds__(Tile<CPLX, G>::THREADS, Tile<CPLX, G>::PER_SM)
+    dmma_gemm_kernel(const DmmaParams p) {
     if (p.guard && *p.guard != 0) return;  // the emulated path produced C
     extern __shared__ __align__(16) double smem[];
-    dmma_tile<CPLX, AKC, BKC, KI, G>(p, blockIdx.x, smem);
+    if (!p.queue) {
+        dmma_tile<CPLX, AKC, BKC, KI, G>(p, blockIdx.x, smem);
+        return;
+    }
+    __shared__ int s_tile;
+    const int tiles = p.tiles_m * p.tiles_n;
+    for (;;) {
+        if (threadIdx.x == 0) s_tile = atomicAdd(p.queue, 1);
+        __syncthreads();
+        const int tile = s_tile;
+        if (tile >= tiles) break;
+        dmma_tile<CPLX, AKC, BKC, KI, G>(p, tile, smem);
+        __syncthreads();  // the next tile's copies reuse the stages, its claim s_tile
+    }
+    // every CTA draws one number past the tiles; the last of them resets the counter
+    if (threadIdx.x == 0 && s_tile == tiles + int(gridDim.x) - 1) atomicExch(p.queue, 0);
+}
+
+// One C tile per cluster, its k extent cut over the cluster's CTAs.
+template <bool CPLX, bool AKC, bool BKC, int KI, int G>
+__global__ void __launch_bounds__(Tile<CPLX, G>::THREADS, Tile<CPLX, G>::PER_SM)
+    dmma_split_kernel(const DmmaParams p, int splits) {
+    if (p.guard && *p.guard != 0) return;  // uniform
+    extern __shared__ __align__(16) double smem[];
+    dmma_tile<CPLX, AKC, BKC, KI, G, true>(p, blockIdx.x / splits, smem, blockIdx.x % splits, splits);
+}
+
+int num_sms() {
+    static const int sms = [] {
+        int dev = 0, n = 148;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+            n = 148;
+        return n;
+    }();
+    return sms;
 }
 
 template <bool CPLX, bool AKC, bool BKC, int KI, int G>
-int launch_cfg(const DmmaParams &p, cudaStream_t s) {
+int launch_cfg(const DmmaParams &p, int splits, cudaStream_t s) {
     using TL = Tile<CPLX, G>;
-    constexpr int PLANES = CPLX ? 2 : 1;
-    constexpr size_t smem = size_t(TL::STAGES) * PLANES *
-                            (SmemOp<TL::BM, TL::BK, AKC>::plane + SmemOp<TL::BN, TL::BK, BKC>::plane) *
-                            sizeof(double);
+    constexpr size_t smem = dmma_smem_bytes<CPLX, AKC, BKC, G>();
     static_assert(smem <= 227 * 1024, "shared memory budget");
+    const int64_t tiles = int64_t(p.tiles_m) * p.tiles_n;
+    if constexpr (G == 2) {
+        if (splits > 1) {
+            auto kern = dmma_split_kernel<CPLX, AKC, BKC, KI, G>;
+            BX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+            BX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            cudaLaunchAttribute at;
+            at.id = cudaLaunchAttributeClusterDimension;
+            at.val.clusterDim.x = unsigned(splits);
+            at.val.clusterDim.y = at.val.clusterDim.z = 1;
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3(unsigned(tiles * splits));
+            cfg.blockDim = dim3(TL::THREADS);
+            cfg.dynamicSmemBytes = smem;
+            cfg.stream = s;
+            cfg.attrs = &at;
+            cfg.numAttrs = 1;
+            BX_CUDA(cudaLaunchKernelEx(&cfg, kern, p, splits));
+            count_launch();
+            return BLASX_OK;
+        }
+    }
     auto kern = dmma_gemm_kernel<CPLX, AKC, BKC, KI, G>;
     BX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    const int64_t tiles = int64_t(p.tiles_m) * p.tiles_n;
-    kern<<<unsigned(tiles), TL::THREADS, smem, s>>>(p);
+    const int64_t grid = p.queue ? std::min<int64_t>(tiles, int64_t(TL::PER_SM) * num_sms()) : tiles;
+    kern<<<unsigned(grid), TL::THREADS, smem, s>>>(p);
     BX_CUDA(cudaGetLastError());
     count_launch();
     return BLASX_OK;
 }
 
-// Instruction K of the FP64 MMA: 16 by default (BLASX_DMMA_K = 4, 8 or 16).
+// Instruction K of the FP64 MMA with the 64x64 and 128x128 tiles: 16 by
+// default (BLASX_DMMA_K = 4, 8 or 16).
 int dmma_k() {
     static const int k = [] {
         const char *e = getenv("BLASX_DMMA_K");
@@ -55,68 +116,102 @@ int dmma_k() {
     return k;
 }
 
-// FP64 CTA geometry, by the estimated fraction of the SMs' FP64 pipes kept
-// busy: a grid of t CTAs, r resident per SM, runs in ceil(t / (r S)) waves,
-// so the busy fraction is t / (ceil(t / (r S)) r S). The 128x128 tile runs
-// one CTA per SM; the 64x64 tile two, at an assumed 85% of the larger
-// tile's per-SM rate (more shared-memory traffic per flop). BLASX_DMMA_TILE
-// = 64 or 128 forces one.
-int dmma_geometry(int64_t M, int64_t N) {
+// The tile geometry and the k split of one problem.
+struct Geometry {
+    int g, splits;
+};
+
+// Chosen by the estimated time in SM cycles. An SM does 64 FP64 multiply-adds
+// per cycle; with n CTAs of a tile resident it reaches the fraction eff[n] of
+// that, measured per tile (few warps cannot cover the shared-memory and
+// barrier latencies: one 64x64 CTA alone reaches 55%, three 87%). A grid runs
+// as full rounds of PER_SM CTAs on every SM and one more with what is left.
+// Cutting k over a cluster costs about 8000 cycles (the exchange of the partial
+// tiles and the cluster launch: 512^3 took 18.6 us with a cut of 2 against
+// 16.6 without), so it is for fewer tiles than SMs with a long k: 96 x 64 x
+// 11904 fell from 590 us (two 64x64 tiles) to 33 with a cut of 8.
+// BLASX_DMMA_TILE = 32, 48 (64x48), 64 or 128 forces an FP64 tile.
+struct TileModel {
+    int g, bm, bn, per_sm;
+    double eff[4];
+};
+constexpr double kSplitCycles = 8000.0;
+constexpr TileModel kReal[] = {{1, 64, 64, 3, {0.55, 0.79, 0.87, 0}},
+                               {3, 64, 48, 4, {0.53, 0.73, 0.77, 0.85}},
+                               {2, 32, 32, 4, {0.43, 0.61, 0.70, 0.774}}};
+constexpr TileModel kCplx[] = {{1, 64, 64, 2, {0.72, 0.86, 0, 0}}, {2, 32, 32, 4, {0.56, 0.76, 0.80, 0.83}}};
+
+template <int COUNT> Geometry pick_geometry(const TileModel (&models)[COUNT], double macs, const Gemm &g) {
+    const int64_t sms = num_sms();
+    Geometry best{models[0].g, 1};
+    double best_t = 1e300;
+    for (const TileModel &m : models) {
+        int64_t tiles = ((g.M + m.bm - 1) / m.bm) * ((g.N + m.bn - 1) / m.bn);
+        if (g.uplo) tiles = (tiles + 1) / 2;  // about half of a triangle's tiles compute
+        const int max_splits = m.g == 2 ? 16 : 1;
+        for (int s = 1; s == 1 || (s <= max_splits && g.K >= int64_t(32) * s && tiles < sms); s *= 2) {
+            const int64_t ctas = tiles * s, round = sms * m.per_sm, rest = ctas % round;
+            const int64_t n = (rest + sms - 1) / sms;
+            const double share = macs * m.bm * m.bn * double((g.K + s - 1) / s) / 64.0;  // one CTA, its pipe to itself
+            const double t = share * (double(ctas / round) * m.per_sm / m.eff[m.per_sm - 1] +
+                                      (n ? double(n) / m.eff[n - 1] : 0.0)) +
+                             (s > 1 ? kSplitCycles : 0.0);
+            if (t < best_t) {
+                best_t = t;
+                best = Geometry{m.g, s};
+            }
+        }
+    }
+    return best;
+}
+
+int forced_tile() {
     static const int forced = [] {
         const char *e = getenv("BLASX_DMMA_TILE");
-        const int v = e ? atoi(e) : 0;
-        return v == 64 ? 1 : (v == 128 ? 0 : -1);
+        switch (e ? atoi(e) : 0) {
+            case 32: return 2;
+            case 48: return 3;
+            case 64: return 1;
+            case 128: return 0;
+            default: return -1;
+        }
     }();
-    if (forced >= 0) return forced;
-    static const int sms = [] {
-        int dev = 0, n = 148;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-            n = 148;
-        return n;
-    }();
-    // share of the SM slots of all waves that hold useful output: occupancy
-    // of the last wave times the part of each tile inside M x N
-    auto useful = [&](int64_t edge, int per_sm) {
-        const int64_t tiles = ((M + edge - 1) / edge) * ((N + edge - 1) / edge);
-        const int64_t slots = int64_t(sms) * per_sm;
-        const int64_t waves = (tiles + slots - 1) / slots;
-        return double(M) * double(N) / (double(waves * slots) * double(edge * edge));
-    };
-    const double big = useful(128, 1);
-    const double small = 0.85 * useful(64, 2);
-    return small > big ? 1 : 0;
+    return forced;
 }
 
-template <bool CPLX, bool AKC, bool BKC, int G> int launch_kg(const DmmaParams &p, cudaStream_t s) {
-    switch (dmma_k()) {
-        case 4: return launch_cfg<CPLX, AKC, BKC, 4, G>(p, s);
-        case 8: return launch_cfg<CPLX, AKC, BKC, 8, G>(p, s);
-        default: return launch_cfg<CPLX, AKC, BKC, 16, G>(p, s);
-    }
-}
-
-template <bool CPLX, bool AKC, bool BKC, int G> int launch_k(const DmmaParams &p, cudaStream_t s) {
-    if constexpr (CPLX) {
-        return launch_cfg<CPLX, AKC, BKC, 4, 0>(p, s);  // complex: register budget
-    } else {
-        return launch_kg<CPLX, AKC, BKC, G>(p, s);
-    }
-}
-
-template <bool CPLX, int G> int launch_g(const Gemm &g, cudaStream_t s) {
+template <bool CPLX, int KI, int G> int launch_g(const Gemm &g, int splits, cudaStream_t s) {
     const DmmaParams p = make_params<CPLX, G>(g);
-    if (int64_t(p.tiles_m) * p.tiles_n > INT32_MAX)
+    if (int64_t(p.tiles_m) * p.tiles_n * splits > INT32_MAX)
         return set_error(BLASX_ERR_UNSUPPORTED, "DMMA grid too large");
     const bool akc = g.ta != NoTrans;  // op(A) = A^T: stored K x M, k contiguous
     const bool bkc = g.tb == NoTrans;  // op(B) = B: stored K x N, k contiguous
-    if (akc) return bkc ? launch_k<CPLX, true, true, G>(p, s) : launch_k<CPLX, true, false, G>(p, s);
-    return bkc ? launch_k<CPLX, false, true, G>(p, s) : launch_k<CPLX, false, false, G>(p, s);
+    if (akc)
+        return bkc ? launch_cfg<CPLX, true, true, KI, G>(p, splits, s) : launch_cfg<CPLX, true, false, KI, G>(p, splits, s);
+    return bkc ? launch_cfg<CPLX, false, true, KI, G>(p, splits, s) : launch_cfg<CPLX, false, false, KI, G>(p, splits, s);
 }
 
-template <bool CPLX> int launch_t(const Gemm &g, cudaStream_t s) {
-    if constexpr (CPLX) return launch_g<CPLX, 0>(g, s);
-    else return dmma_geometry(g.M, g.N) == 1 ? launch_g<CPLX, 1>(g, s) : launch_g<CPLX, 0>(g, s);
+template <int G> int launch_k(const Gemm &g, cudaStream_t s) {
+    switch (dmma_k()) {
+        case 4: return launch_g<false, 4, G>(g, 1, s);
+        case 8: return launch_g<false, 8, G>(g, 1, s);
+        default: return launch_g<false, 16, G>(g, 1, s);
+    }
+}
+
+int launch_real(const Gemm &g, cudaStream_t s) {
+    Geometry x = pick_geometry(kReal, 1.0, g);
+    if (forced_tile() >= 0) x = Geometry{forced_tile(), 1};
+    switch (x.g) {
+        case 0: return launch_k<0>(g, s);
+        case 1: return launch_k<1>(g, s);
+        case 3: return launch_g<false, 16, 3>(g, 1, s);
+        default: return launch_g<false, 16, 2>(g, x.splits, s);
+    }
+}
+
+int launch_cplx(const Gemm &g, cudaStream_t s) {
+    const Geometry x = pick_geometry(kCplx, 4.0, g);
+    return x.g == 1 ? launch_g<true, 8, 1>(g, 1, s) : launch_g<true, 4, 2>(g, x.splits, s);
 }
 
 }  // namespace
@@ -127,8 +222,8 @@ bool dmma_supported(const Gemm &g) {
 }
 
 int launch_gemm_dmma(const Gemm &g, cudaStream_t s) {
-    if (g.dt == DType::F64) return launch_t<false>(g, s);
-    if (g.dt == DType::C128) return launch_t<true>(g, s);
+    if (g.dt == DType::F64) return launch_real(g, s);
+    if (g.dt == DType::C128) return launch_cplx(g, s);
     return set_error(BLASX_ERR_UNSUPPORTED, "DMMA kernel handles FP64 and complex128 only");
 }
 

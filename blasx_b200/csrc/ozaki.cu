@@ -199,6 +199,7 @@ int ozaki_run(const Gemm &g, cudaStream_t s, int mode, void *ws, int num_sms, vo
             gp.C = static_cast<char *>(g.C) + j0 * g.ldc * int64_t(elem_size(g.dt));
             gp.diag = g.diag + j0;
             gp.guard = &dec->nmod;
+            gp.queue = &dec->pad;
             if (dmma_supported(gp)) BX_TRY(launch_gemm_dmma(gp, s));
             else BX_TRY(launch_gemm_simt(gp, s));
         }
@@ -211,6 +212,7 @@ int ozaki_run(const Gemm &g, cudaStream_t s, int mode, void *ws, int num_sms, vo
     if (!hooks) {
         Gemm gn = g;
         gn.guard = &dec->nmod;
+        gn.queue = &dec->pad;
         if (dmma_supported(gn)) BX_TRY(launch_gemm_dmma(gn, s));
         else BX_TRY(launch_gemm_simt(gn, s));
     }

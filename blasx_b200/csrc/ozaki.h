@@ -46,7 +46,7 @@ struct Decision {
     int q;         // norm exponent bound Q
     double estimate;  // estimated max normalised error (units of the dtype's u)
     int nonfinite;
-    int pad;
+    int pad;  // zero; arrival counter before the decision, tile counter of the fallback after it
 };
 
 // Row/column statistics of one operand (R rows of op(X), each over K).

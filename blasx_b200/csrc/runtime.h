@@ -55,6 +55,9 @@ struct Gemm {
     // Device pointer; when set, the native kernels return at once unless
     // *guard == 0 (the emulated path chose its native fallback on the device).
     const int *guard = nullptr;
+    // With guard: a device word, zero between launches, from which a
+    // tensor-pipe kernel with fewer CTAs than tiles hands out its tiles.
+    int *queue = nullptr;
     // Emulated path: at most this many residue-GEMM tiles per CTA (0: one
     // persistent CTA per SM). A bound makes its CTAs retire every few
     // milliseconds, so that kernels of other streams get SMs in between.
