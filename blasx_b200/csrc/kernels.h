@@ -20,8 +20,8 @@ int launch_real_diagonal(DType dt, void *C, int64_t ldc, int64_t m, int64_t n, i
 // g.C (g.M x g.N, ld g.ldc) += g.beta * X (ld ldx); nothing when beta == 0.
 int launch_add_scaled(const Gemm &g, const void *X, int64_t ldx, cudaStream_t s);
 
-// Portable SIMT tiled kernel (all dtypes, transposes, ragged edges). Used for
-// small problems and as the first correct path.
+// FP32 and complex64 on the CUDA cores (fma_preferred), and the portable SIMT
+// tiled kernel for what is left (large complex64, all dtypes).
 int launch_gemm_simt(const Gemm &g, cudaStream_t s);
 
 // Native FP64 / complex128 kernel on the FP64 tensor pipe (DMMA).
@@ -32,10 +32,10 @@ bool dmma_supported(const Gemm &g);
 // Device-resident GEMM of any dtype through the best available path.
 // Uses library-owned scratch memory for the Ozaki path.
 int device_gemm(const Gemm &g, cudaStream_t s);
-// FP32 on the CUDA cores with a 128 x 128 tile per CTA, for problems of at
-// least one wave of such tiles (launch_gemm_simt picks it by sgemm128_fits).
-bool sgemm128_fits(const Gemm &g);
-int launch_sgemm128(const Gemm &g, cudaStream_t s);
+// FP32 / complex64 on the CUDA cores with tiles chosen by size (launch_gemm_simt
+// takes it where fma_preferred).
+bool fma_preferred(const Gemm &g);
+int launch_gemm_fma(const Gemm &g, cudaStream_t s);
 // Triangular solve on device operands (t.A, t.B device pointers): recursive
 // halving into device_gemm updates (native or emulated by the precision
 // mode) and a substitution kernel for blocks of <= 64 rows. Sets *emulated
