@@ -18,6 +18,7 @@ template <typename T> struct Arith;
 
 template <> struct Arith<float> {
     using V = float;
+    using R = float;  // real scalar
     __device__ static V zero() { return 0.f; }
     __device__ static V one() { return 1.f; }
     __device__ static V real_part(V a) { return a; }
@@ -28,6 +29,7 @@ template <> struct Arith<float> {
 };
 template <> struct Arith<double> {
     using V = double;
+    using R = double;  // real scalar
     __device__ static V zero() { return 0.0; }
     __device__ static V one() { return 1.0; }
     __device__ static V real_part(V a) { return a; }
@@ -38,6 +40,7 @@ template <> struct Arith<double> {
 };
 template <> struct Arith<z2> {
     using V = z2;
+    using R = double;  // real scalar
     __device__ static V zero() { return {0.0, 0.0}; }
     __device__ static V one() { return {1.0, 0.0}; }
     __device__ static V real_part(V a) { return {a.re, 0.0}; }
@@ -57,6 +60,7 @@ template <> struct Arith<z2> {
 
 template <> struct Arith<c2> {
     using V = c2;
+    using R = float;  // real scalar
     __device__ static V zero() { return {0.f, 0.f}; }
     __device__ static V one() { return {1.f, 0.f}; }
     __device__ static V real_part(V a) { return {a.re, 0.f}; }

@@ -38,7 +38,7 @@ bool fma_preferred(const Gemm &g);
 int launch_gemm_fma(const Gemm &g, cudaStream_t s);
 // Triangular solve on device operands (t.A, t.B device pointers): recursive
 // halving into device_gemm updates (native or emulated by the precision
-// mode) and a substitution kernel for blocks of <= 64 rows. Sets *emulated
+// mode) and a substitution kernel for blocks of <= 256 rows. Sets *emulated
 // when any update took the emulated path.
 int trsm_device(const Trsm &t, cudaStream_t s, bool *emulated);
 // The largest update GEMM trsm_device issues for t (its scratch bounds the

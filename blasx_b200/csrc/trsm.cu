@@ -7,7 +7,7 @@
 // emulated on the INT8 tensor cores where the precision mode selects it),
 // solve the second half. The top-level updates carry most of the K^2 * (M or
 // N) work with K up to K/2, the shape the emulated GEMM needs; blocks of at
-// most 64 rows (32 complex) are solved by substitution in one kernel.
+// most 256 rows are solved by substitution in one kernel.
 //
 // Every GEMM reads op(A) only in an off-diagonal rectangle inside the stored
 // triangle, and the substitution kernel reads only the stored triangle of its
@@ -21,22 +21,17 @@
 namespace bx {
 namespace {
 
-// Order of a substitution block: one right-hand-side vector of it lives in
-// one thread's registers (64 doubles, or 32 complex doubles).
-template <typename T> struct LeafDim {
-    static constexpr int n = 64;
+// Geometry of the substitution kernel. A warp holds a few right-hand-side
+// vectors of a block of kBlock rows in registers: lane l owns rows l, l + 32,
+// ... of each.
+constexpr int kBlock = 256, kRows = kBlock / 32;
+constexpr int kBlockThreads = 256;
+constexpr int kPanel = 16;  // columns of S staged at a time
+constexpr int kPanelLd = kBlock + 1;
+// Vectors per warp: 16 bytes of each row per lane (32 registers in all).
+template <typename T> struct Vecs {
+    static constexpr int n = 16 / int(sizeof(T));
 };
-template <> struct LeafDim<z2> {
-    static constexpr int n = 32;
-};
-template <> struct LeafDim<c2> {
-    static constexpr int n = 32;
-};
-constexpr int kLeafVecs = 64;     // right-hand-side vectors per CTA
-constexpr int kLanes = 4;         // lanes per vector: lane j owns rows j, j + 4, ...
-constexpr int kLeafThreads = kLeafVecs * kLanes;
-
-int leaf_order(DType dt) { return is_complex(dt) ? 32 : 64; }
 
 template <typename T> __device__ inline T negate(T a) { return -a; }
 template <> __device__ inline z2 negate<z2>(z2 a) { return {-a.re, -a.im}; }
@@ -50,7 +45,19 @@ template <> __device__ inline c2 shfl<c2>(c2 v, int src) {
     return {__shfl_sync(0xffffffffu, v.re, src), __shfl_sync(0xffffffffu, v.im, src)};
 }
 
-// Solves S x = c for nvec vectors at once, S the bs x bs (bs <= L) system
+// One scalar of shared memory from global memory, or zero.
+template <typename T> __device__ __forceinline__ void copy_or_zero(T *dst, const T *src, bool in) {
+    using R = typename Arith<T>::R;
+    constexpr int RW = int(sizeof(R)), PARTS = int(sizeof(T)) / RW;
+#pragma unroll
+    for (int q = 0; q < PARTS; ++q)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %3, %2;\n" ::"r"(
+                         uint32_t(__cvta_generic_to_shared(dst)) + q * RW),
+                     "l"(reinterpret_cast<const char *>(src) + q * RW), "r"(in ? RW : 0), "n"(RW)
+                     : "memory");
+}
+
+// Solves S x = c for nvec vectors at once, S the bs x bs (bs <= kBlock) system
 // matrix of one diagonal block: S = op(A_block) for a left solve, the
 // transpose of op(A_block) for a right solve (x op(A) = c is op(A)^T x^T =
 // c^T). S[i][k] is A[i + k lda] (s_trans = 0) or A[k + i lda] (s_trans = 1),
@@ -59,127 +66,169 @@ template <> __device__ inline c2 shfl<c2>(c2 v, int src) {
 // element i: left: C[i + v ldc] (columns of B); right: C[v + i ldc] (rows of
 // B). Each vector is scaled by `scale` (alpha) on load.
 //
-// Shared memory holds S by columns (St[k * L + i] = S[i][k]), zero outside
-// the triangle, the reciprocals of its diagonal and, for a left solve, the
-// CTA's vectors: they are columns of B, which consecutive threads load and
-// store row by row (coalesced) through shared memory. Four adjacent lanes
-// solve one vector held in their registers, lane j owning rows j, j + 4, ...
-// The substitution is unrolled over the L x L block, so every register index
-// is a compile-time constant; at step k the lane owning row k scales it by
-// 1 / S[k][k], a shuffle hands x_k to the other three, and each lane updates
-// its later rows (no barrier). A block smaller than L is padded with zero
-// right-hand sides and unit diagonal, which leave the real rows unchanged.
+// What bounds it: the chain of bs dependent steps of each vector (a
+// reciprocal multiply, a shuffle and a multiply-add, ~60 cycles), and beside
+// it the FP64 pipe. So a block is as tall as its vectors fit in registers, one
+// launch instead of four substitutions of 64 rows with three updates between
+// them; every warp runs its own vectors, the rows after step k updated by all
+// lanes at once, and a step needs no barrier. S passes through shared memory
+// 16 columns at a time (cp.async, the next panel in flight), zero outside its
+// triangle and beyond bs; the CTA's warps share it. Rows beyond bs are zero
+// vectors with a unit diagonal. FP64, 256 rows: 28.5 us for 2048 vectors (87
+// as four 64-row substitutions and their updates), 132 for 16384 (136); a
+// DTRSM of 4096 rows and 2048 vectors fell from 2083 to 1417 us. Four vectors
+// per lane and four warps per CTA took 79 us for 2048: with one warp per
+// scheduler every instruction's latency shows.
 template <typename T, bool FORWARD, bool UNIT>
-__global__ void __launch_bounds__(kLeafThreads)
-    trsm_leaf_kernel(const T *__restrict__ A, int64_t lda, T *__restrict__ C, int64_t ldc, int bs,
-                     int64_t nvec, int left, int s_trans, int s_conj, T scale) {
+__global__ void __launch_bounds__(kBlockThreads)
+    trsm_block_kernel(const T *__restrict__ A, int64_t lda, T *__restrict__ C, int64_t ldc, int bs, int64_t nvec,
+                      int left, int s_trans, int s_conj, T scale) {
     using Ar = Arith<T>;
-    constexpr int L = LeafDim<T>::n;
-    constexpr int R = L / kLanes;  // rows per lane
+    constexpr int NV = Vecs<T>::n, TH = kBlockThreads, WARPS = TH / 32;
+    static_assert(TH == kBlock, "a thread loads one row of a panel");
     extern __shared__ __align__(16) unsigned char smem[];
-    T *St = reinterpret_cast<T *>(smem);  // St[k * L + i] = S[i][k]
-    T *rdiag = St + L * L;                // 1 / S[k][k]
-    T *Cs = rdiag + L;                    // left: Cs[v * (L + 1) + i], this CTA's vectors
-    const int64_t v0 = int64_t(blockIdx.x) * kLeafVecs;
-    const int tid = threadIdx.x;
-    // global -> shared: every load of a thread is issued before its stores
-    constexpr int kStPer = L * L / kLeafThreads, kCsPer = L * kLeafVecs / kLeafThreads;
-    static_assert(kStPer * kLeafThreads == L * L && kCsPer * kLeafThreads == L * kLeafVecs, "whole batches");
-    if (left) {  // a left vector is a column of B: consecutive threads take consecutive rows
-        T tmp[kCsPer];
+    T *P = reinterpret_cast<T *>(smem);            // P[buf][k][i]: S[i][k0 + k]
+    T *rdiag = P + 2 * kPanel * kPanelLd;          // 1 / S[k][k]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t v0 = (int64_t(blockIdx.x) * WARPS + warp) * NV;
+
+    // panel at column k0 of S into buffer b. Untransposed: thread i copies
+    // row i, column after column (coalesced); transposed: 16 threads a row's
+    // 16 columns. Rows of 32-row groups that the panel's steps do not read
+    // are skipped.
+    auto load_panel = [&](int k0, int b) {
+        T *dst = P + b * kPanel * kPanelLd;
+        const int g = k0 / 32 * 32;
+        if (!s_trans) {
+            const int i = tid;
+            if (FORWARD ? i >= g : i < g + 32) {
+                const T *src = A + i + int64_t(k0) * lda;
 #pragma unroll
-        for (int q = 0; q < kCsPer; ++q) {
-            const int e = tid + q * kLeafThreads, i = e % L, vv = e / L;
-            tmp[q] = (i < bs && v0 + vv < nvec) ? C[i + (v0 + vv) * ldc] : Ar::zero();
+                for (int k = 0; k < kPanel; ++k, src += lda) {
+                    const bool in = i < bs && k0 + k < bs && (FORWARD ? i > k0 + k : i < k0 + k);
+                    copy_or_zero(dst + k * kPanelLd + i, in ? src : A, in);
+                }
+            }
+        } else {
+            const int k = tid % kPanel, col = k0 + k;
+            const int i0 = (FORWARD ? g : 0) + tid / kPanel, i1 = FORWARD ? kBlock : g + 32;
+            const T *src = A + col + int64_t(i0) * lda;
+#pragma unroll 2
+            for (int i = i0; i < i1; i += TH / kPanel, src += int64_t(TH / kPanel) * lda) {
+                const bool in = i < bs && col < bs && (FORWARD ? i > col : i < col);
+                copy_or_zero(dst + k * kPanelLd + i, in ? src : A, in);
+            }
         }
-#pragma unroll
-        for (int q = 0; q < kCsPer; ++q) {
-            const int e = tid + q * kLeafThreads;
-            Cs[(e / L) * (L + 1) + e % L] = tmp[q];
-        }
-    }
-    {
-        T tmp[kStPer];
-#pragma unroll
-        for (int q = 0; q < kStPer; ++q) {
-            const int e = tid + q * kLeafThreads, i = e % L, k = e / L;
-            tmp[q] = Ar::zero();
-            if (i < bs && k < bs && (FORWARD ? i > k : i < k))
-                tmp[q] = s_trans ? A[k + int64_t(i) * lda] : A[i + int64_t(k) * lda];
-        }
-#pragma unroll
-        for (int q = 0; q < kStPer; ++q) St[tid + q * kLeafThreads] = s_conj ? Ar::conj(tmp[q]) : tmp[q];
-    }
-    if (tid < L) {
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    const int first = FORWARD ? 0 : (bs - 1) / kPanel * kPanel;
+    load_panel(first, first / kPanel & 1);
+    for (int i = tid; i < kBlock; i += TH) {
         T r = Ar::one();
-        if (!UNIT && tid < bs) {
-            T d = A[tid + int64_t(tid) * lda];
+        if (!UNIT && i < bs) {
+            T d = A[i + int64_t(i) * lda];
             if (s_conj) d = Ar::conj(d);
             r = quot(Ar::one(), d);
         }
-        rdiag[tid] = r;
+        rdiag[i] = r;
     }
-    __syncthreads();
-    const int j = tid % kLanes, vl = tid / kLanes;
-    const int64_t v = v0 + vl;
-    const bool live = v < nvec;
-    const int base = tid & ~(kLanes - 1);  // lane 0 of this vector's group
-    T c[R];
+    // c[m]: minus the sum of S[i][k] x_k so far, until group m's turn; then
+    // its right-hand sides are added in one rounding (a running subtraction
+    // from them would round at their size at every step) and it is solved
+    T c[kRows][NV], rhs[NV];
 #pragma unroll
-    for (int m = 0; m < R; ++m) {
-        const int i = j + kLanes * m;
-        c[m] = Ar::zero();
-        if (i < bs && live) c[m] = Ar::mul(scale, left ? Cs[vl * (L + 1) + i] : C[v + int64_t(i) * ldc]);
-    }
+    for (int m = 0; m < kRows; ++m)
 #pragma unroll
-    for (int s = 0; s < L; ++s) {
-        const int k = FORWARD ? s : L - 1 - s;
-        const int mk = k / kLanes, jk = k % kLanes;
-        if (!UNIT && j == jk) c[mk] = Ar::mul(c[mk], rdiag[k]);
-        const T xk = shfl(c[mk], base + jk);
-        const T *col = St + k * L;
+        for (int v = 0; v < NV; ++v) c[m][v] = Ar::zero();
+    auto load_rhs = [&](int m) {
+        const int i = lane + 32 * m;
 #pragma unroll
-        for (int m = 0; m < R; ++m) {
-            const int i = j + kLanes * m;
-            if (FORWARD ? (kLanes * m + kLanes - 1 > k && i > k) : (kLanes * m < k && i < k))
-                c[m] = Ar::fma(negate(col[i]), xk, c[m]);
+        for (int v = 0; v < NV; ++v) {
+            rhs[v] = Ar::zero();
+            if (i < bs && v0 + v < nvec) rhs[v] = left ? C[i + (v0 + v) * ldc] : C[v0 + v + int64_t(i) * ldc];
+        }
+    };
+    load_rhs(FORWARD ? 0 : (bs - 1) / 32);
+
+#pragma unroll
+    for (int mm = 0; mm < kRows; ++mm) {
+        const int m = FORWARD ? mm : kRows - 1 - mm;  // compile-time after unrolling
+        if (32 * m >= bs) continue;
+#pragma unroll
+        for (int v = 0; v < NV; ++v) c[m][v] = Ar::add(Ar::mul(scale, rhs[v]), c[m][v]);
+        if (FORWARD ? 32 * (m + 1) < bs : m > 0) load_rhs(FORWARD ? m + 1 : m - 1);
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h) {
+            const int half = FORWARD ? h : 1 - h, k0 = 32 * m + 16 * half;
+            if (k0 >= bs) continue;
+            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+            __syncthreads();  // the panel has landed, and every warp has left the other buffer
+            const int next = FORWARD ? k0 + kPanel : k0 - kPanel;
+            if (FORWARD ? next < bs : next >= 0) load_panel(next, next / kPanel & 1);
+            const T *panel = P + (k0 / kPanel & 1) * kPanel * kPanelLd + lane;
+#pragma unroll 4
+            for (int q = 0; q < kPanel; ++q) {
+                const int kq = FORWARD ? q : kPanel - 1 - q;
+                const int kk = 16 * half + kq;  // the lane owning row k
+                const T *col = panel + kq * kPanelLd;
+                T x[NV];
+#pragma unroll
+                for (int v = 0; v < NV; ++v) {
+                    const T s = UNIT ? c[m][v] : Ar::mul(c[m][v], rdiag[k0 + kq]);
+                    x[v] = shfl(s, kk);
+                }
+                const bool after = FORWARD ? lane > kk : lane < kk;
+                {
+                    T s = col[32 * m];
+                    if (s_conj) s = Ar::conj(s);
+                    s = negate(s);
+#pragma unroll
+                    for (int v = 0; v < NV; ++v)
+                        if (after) c[m][v] = Ar::fma(s, x[v], c[m][v]);
+                }
+#pragma unroll
+                for (int r = 0; r < kRows; ++r) {
+                    if (FORWARD ? r <= m : r >= m) continue;
+                    T s = col[32 * r];
+                    if (s_conj) s = Ar::conj(s);
+                    s = negate(s);
+#pragma unroll
+                    for (int v = 0; v < NV; ++v) c[r][v] = Ar::fma(s, x[v], c[r][v]);
+                }
+            }
         }
     }
-    if (!left) {
-        if (live)
 #pragma unroll
-            for (int m = 0; m < R; ++m) {
-                const int i = j + kLanes * m;
-                if (i < bs) C[v + int64_t(i) * ldc] = c[m];
+    for (int m = 0; m < kRows; ++m)
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            const int i = lane + 32 * m;
+            if (i < bs && v0 + v < nvec) {
+                // x_i: the same product that went to the other lanes at step i
+                if (!UNIT) c[m][v] = Ar::mul(c[m][v], rdiag[i]);
+                if (left) C[i + (v0 + v) * ldc] = c[m][v];
+                else C[v0 + v + int64_t(i) * ldc] = c[m][v];
             }
-        return;
-    }
-#pragma unroll
-    for (int m = 0; m < R; ++m) Cs[vl * (L + 1) + j + kLanes * m] = c[m];
-    __syncthreads();
-    for (int e = tid; e < L * kLeafVecs; e += kLeafThreads) {
-        const int i = e % L, vv = e / L;
-        if (i < bs && v0 + vv < nvec) C[i + (v0 + vv) * ldc] = Cs[vv * (L + 1) + i];
-    }
+        }
 }
 
-template <typename T> size_t leaf_smem() {
-    constexpr int L = LeafDim<T>::n;
-    return sizeof(T) * (L * (L + 1) + kLeafVecs * (L + 1));
+template <typename T> constexpr size_t block_smem() {
+    return sizeof(T) * (2 * kPanel * kPanelLd + kBlock);
 }
 
 template <typename T, bool FORWARD, bool UNIT>
-int launch_leaf_k(const Trsm &t, int64_t lo, int64_t hi, cplx scale, int s_trans, cudaStream_t s) {
+int launch_block_k(const Trsm &t, int64_t lo, int64_t hi, cplx scale, int s_trans, cudaStream_t s) {
     static const cudaError_t attr = cudaFuncSetAttribute(
-        trsm_leaf_kernel<T, FORWARD, UNIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(leaf_smem<T>()));
+        trsm_block_kernel<T, FORWARD, UNIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(block_smem<T>()));
     BX_CUDA(attr);
     const int64_t nvec = t.left ? t.N : t.M;
     const T *A = static_cast<const T *>(t.A) + lo + lo * t.lda;
     T *C = static_cast<T *>(t.B) + (t.left ? lo : lo * t.ldb);
-    const int64_t blocks = (nvec + kLeafVecs - 1) / kLeafVecs;
+    constexpr int per = kBlockThreads / 32 * Vecs<T>::n;
+    const int64_t blocks = (nvec + per - 1) / per;
     if (blocks > 0x7fffffff) return set_error(BLASX_ERR_UNSUPPORTED, "trsm: too many right-hand sides");
     const bool conj = is_complex(t.dt) && t.trans == ConjT;
-    trsm_leaf_kernel<T, FORWARD, UNIT><<<unsigned(blocks), kLeafThreads, leaf_smem<T>(), s>>>(
+    trsm_block_kernel<T, FORWARD, UNIT><<<unsigned(blocks), kBlockThreads, block_smem<T>(), s>>>(
         A, t.lda, C, t.ldb, int(hi - lo), nvec, t.left, s_trans, conj, from_cplx<T>(scale));
     BX_CUDA(cudaGetLastError());
     count_launch();
@@ -187,20 +236,20 @@ int launch_leaf_k(const Trsm &t, int64_t lo, int64_t hi, cplx scale, int s_trans
 }
 
 template <typename T>
-int launch_leaf_t(const Trsm &t, int64_t lo, int64_t hi, cplx scale, int s_trans, int forward, cudaStream_t s) {
+int launch_block_t(const Trsm &t, int64_t lo, int64_t hi, cplx scale, int s_trans, int forward, cudaStream_t s) {
     if (forward)
-        return t.unit ? launch_leaf_k<T, true, true>(t, lo, hi, scale, s_trans, s)
-                      : launch_leaf_k<T, true, false>(t, lo, hi, scale, s_trans, s);
-    return t.unit ? launch_leaf_k<T, false, true>(t, lo, hi, scale, s_trans, s)
-                  : launch_leaf_k<T, false, false>(t, lo, hi, scale, s_trans, s);
+        return t.unit ? launch_block_k<T, true, true>(t, lo, hi, scale, s_trans, s)
+                      : launch_block_k<T, true, false>(t, lo, hi, scale, s_trans, s);
+    return t.unit ? launch_block_k<T, false, true>(t, lo, hi, scale, s_trans, s)
+                  : launch_block_k<T, false, false>(t, lo, hi, scale, s_trans, s);
 }
 
-int launch_leaf(const Trsm &t, int64_t lo, int64_t hi, cplx scale, int s_trans, int forward, cudaStream_t s) {
+int launch_block(const Trsm &t, int64_t lo, int64_t hi, cplx scale, int s_trans, int forward, cudaStream_t s) {
     switch (t.dt) {
-        case DType::F32: return launch_leaf_t<float>(t, lo, hi, scale, s_trans, forward, s);
-        case DType::F64: return launch_leaf_t<double>(t, lo, hi, scale, s_trans, forward, s);
-        case DType::C64: return launch_leaf_t<c2>(t, lo, hi, scale, s_trans, forward, s);
-        default: return launch_leaf_t<z2>(t, lo, hi, scale, s_trans, forward, s);
+        case DType::F32: return launch_block_t<float>(t, lo, hi, scale, s_trans, forward, s);
+        case DType::F64: return launch_block_t<double>(t, lo, hi, scale, s_trans, forward, s);
+        case DType::C64: return launch_block_t<c2>(t, lo, hi, scale, s_trans, forward, s);
+        default: return launch_block_t<z2>(t, lo, hi, scale, s_trans, forward, s);
     }
 }
 
@@ -209,16 +258,16 @@ struct Range {
     int64_t size() const { return hi - lo; }
 };
 
-// The system matrix S of the blocks (see trsm_leaf_kernel) is A or A^T:
+// The system matrix S of the blocks (see trsm_block_kernel) is A or A^T:
 // s_trans = 1 when S = A^T. Substitution runs forward when S is lower.
 int s_trans_of(const Trsm &t) { return t.left ? t.trans != NoTrans : t.trans == NoTrans; }
 bool forward_of(const Trsm &t) { return t.lower != bool(s_trans_of(t)); }
 
 // The two halves of [lo, hi) in solve order: the first has a multiple of
-// the leaf order rows.
+// kBlock rows.
 void split(const Trsm &t, Range r, Range *first, Range *second) {
-    const int64_t n = r.size(), lf = leaf_order(t.dt);
-    const int64_t half = std::min(n - 1, (n / 2 + lf - 1) / lf * lf);
+    const int64_t n = r.size();
+    const int64_t half = std::min(n - 1, (n / 2 + kBlock - 1) / kBlock * kBlock);
     if (forward_of(t)) {
         *first = {r.lo, r.lo + half};
         *second = {r.lo + half, r.hi};
@@ -268,7 +317,7 @@ Gemm update_gemm(const Trsm &t, Range tgt, Range src, cplx alpha, cplx beta) {
 constexpr cplx kMinusOne{-1.0, 0.0}, kOne{1.0, 0.0};
 
 int solve(const Trsm &t, Range r, cplx scale, cudaStream_t s, bool *emulated) {
-    if (r.size() <= leaf_order(t.dt)) return launch_leaf(t, r.lo, r.hi, scale, s_trans_of(t), forward_of(t), s);
+    if (r.size() <= kBlock) return launch_block(t, r.lo, r.hi, scale, s_trans_of(t), forward_of(t), s);
     Range first, second;
     split(t, r, &first, &second);
     BX_TRY(solve(t, first, scale, s, emulated));
@@ -410,7 +459,7 @@ int trsm_update_part(const Trsm &t, int64_t tgt_lo, int64_t tgt_hi, int64_t src_
 
 Gemm trsm_top_update(const Trsm &t) {
     const Range all{0, t.order()};
-    if (all.size() <= leaf_order(t.dt)) {
+    if (all.size() <= kBlock) {
         Gemm g = update_gemm(t, all, all, kMinusOne, t.alpha);
         g.K = 0;
         return g;
