@@ -44,6 +44,28 @@ __global__ void __launch_bounds__(256, ROLE == 0 ? 4 : (ROLE == 1 ? 3 : 2)) slic
     slice_rc_body<T, ROLE>(v, st, dec, expo, o, blockIdx.x, blockIdx.y, threadIdx.x, smem);
 }
 
+// Both operands of a real GEMM: blocks [0, na) slice op(A), the others op(B).
+struct SliceSide {
+    View v;
+    RowStats st;
+    int *expo;
+    SliceOut o;
+    int gx;  // blocks along k
+};
+template <typename T, bool AKC, bool BKC>
+__global__ void __launch_bounds__(256, 4) slice_both_kernel(SliceSide a, SliceSide b, int na, const Decision *dec) {
+    __shared__ __align__(16) unsigned char smem[(AKC && BKC) ? 16 : slice_rc_smem_bytes<0>()];
+    const int i = blockIdx.x;
+    if (i < na) {
+        if (AKC) slice_kc_body<T, 0>(a.v, a.st, dec, a.expo, a.o, i % a.gx, i / a.gx, threadIdx.x);
+        else slice_rc_body<T, 0>(a.v, a.st, dec, a.expo, a.o, i % a.gx, i / a.gx, threadIdx.x, smem);
+    } else {
+        const int j = i - na;
+        if (BKC) slice_kc_body<T, 0>(b.v, b.st, dec, b.expo, b.o, j % b.gx, j / b.gx, threadIdx.x);
+        else slice_rc_body<T, 0>(b.v, b.st, dec, b.expo, b.o, j % b.gx, j / b.gx, threadIdx.x, smem);
+    }
+}
+
 template <typename T, bool CPLX>
 __global__ void __launch_bounds__(128) reconstruct_kernel(const ReconArgs a, const Decision *dec) {
     reconstruct_body<T, CPLX>(a, dec, blockIdx.x, blockIdx.y, threadIdx.x);
@@ -119,6 +141,32 @@ int launch_slice(const oz::View &v, bool kc, const oz::RowStats &st, const oz::D
     return BLASX_OK;
 }
 
+// Both operands of a real GEMM in one launch (one tail instead of two: at
+// 2048^3 an operand alone is 1.7 waves of blocks). False when the grid would
+// be too large.
+template <typename T>
+bool slice_both_fits(const oz::SliceOut &oa, const oz::SliceOut &ob, int64_t Kc) {
+    return (Kc / 64) * (oa.Rp / 64 + ob.Rp / 64) <= INT32_MAX;
+}
+template <typename T>
+int launch_slice_both(const oz::View &va, bool akc, const oz::RowStats &sa, int *ea, const oz::SliceOut &oa,
+                      const oz::View &vb, bool bkc, const oz::RowStats &sb, int *fb, const oz::SliceOut &ob,
+                      const oz::Decision *dec, int64_t Kc, cudaStream_t s) {
+    const int gx = int(Kc / 64), na = int(gx * (oa.Rp / 64)), nb = int(gx * (ob.Rp / 64));
+    const oz::SliceSide a{va, sa, ea, oa, gx}, b{vb, sb, fb, ob, gx};
+    const unsigned grid = unsigned(na) + unsigned(nb);
+    if (akc) {
+        if (bkc) oz::slice_both_kernel<T, true, true><<<grid, 256, 0, s>>>(a, b, na, dec);
+        else oz::slice_both_kernel<T, true, false><<<grid, 256, 0, s>>>(a, b, na, dec);
+    } else {
+        if (bkc) oz::slice_both_kernel<T, false, true><<<grid, 256, 0, s>>>(a, b, na, dec);
+        else oz::slice_both_kernel<T, false, false><<<grid, 256, 0, s>>>(a, b, na, dec);
+    }
+    BX_CUDA(cudaGetLastError());
+    count_launch();
+    return BLASX_OK;
+}
+
 // The whole emulated pipeline on a caller-provided workspace of
 // make_plan(g).bytes bytes: no allocation. The device decision and error
 // flag are copied to the given host slots when they are not null.
@@ -156,8 +204,12 @@ int ozaki_run(const Gemm &g, cudaStream_t s, int mode, void *ws, int num_sms, vo
         BX_TRY((launch_slice<T, 1>(va, akc, sa, dec, ea, oy, Kc, s)));
         BX_TRY((launch_slice<T, 2>(vb, bkc, sb, dec, fb, ox, Kc, s)));
     } else {
-        BX_TRY((launch_slice<T, 0>(va, akc, sa, dec, ea, oy, Kc, s)));
-        if (!pl.alias) BX_TRY((launch_slice<T, 0>(vb, bkc, sb, dec, fb, ox, Kc, s)));
+        if (!pl.alias && slice_both_fits<T>(oy, ox, Kc)) {
+            BX_TRY(launch_slice_both<T>(va, akc, sa, ea, oy, vb, bkc, sb, fb, ox, dec, Kc, s));
+        } else {
+            BX_TRY((launch_slice<T, 0>(va, akc, sa, dec, ea, oy, Kc, s)));
+            if (!pl.alias) BX_TRY((launch_slice<T, 0>(vb, bkc, sb, dec, fb, ox, Kc, s)));
+        }
     }
     // residue GEMMs and reconstruction, in column panels of C when asked.
     // (Running a panel's reconstruction on a second stream beside the next

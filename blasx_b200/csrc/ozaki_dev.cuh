@@ -322,6 +322,12 @@ template <int L> struct Mod {
     static constexpr uint32_t magic = uint32_t(((uint64_t(1) << 32) + m - 1) / m);
     // h * magic: (s + h) * magic as one 64-bit multiply-add of s
     static constexpr uint64_t hmagic = uint64_t(h) * magic;
+    // FP32 reduction: a multiple of 256 m at or above 1.5 * 2^23, its quotient,
+    // and the bits of the float of that value plus cb
+    static constexpr uint32_t base = 256 * m * ((12582912u + 256 * m - 1) / (256 * m));
+    static constexpr uint32_t base_q = base / m;
+    static constexpr uint32_t fbits = 0x4B000000u + (base - 8388608u) + cb;
+    static_assert(base + 8 * 255 * 255 + 255 < (1u << 24), "base + s is an exact float");
 };
 
 // v + 2^62 (|v| < 2^62, so the biased value is in [0, 2^63)) as two 32-bit
@@ -334,26 +340,57 @@ __device__ __forceinline__ Digits digits_of(int64_t v) {
     return {uint32_t(a), uint32_t(a >> 32)};
 }
 
-// Symmetric residue of v for the L-th modulus, in [-h, h] for odd m (the
-// low byte for m = 256, whose byte is already the two's complement of the
-// residue in [-128, 127]): with the bias removed, the bytes b_k of the
-// biased value give
+// Residue of v for the L-th modulus, its low byte an int8 in [-127, 127] (the
+// byte itself, the two's complement of [-128, 127], for m = 256): with the
+// bias removed, the bytes b_k of the biased value give
 //   s = sum_k b_k (2^(8k) mod m) + (-2^62 mod m) <= 8 * 255 * 255 + 255,
 // two byte dot products (DP4A) against constant weight words, s = v (mod m).
-// With t = s + h < 2^20,
-//   q = floor(t / m) = floor(t ceil(2^32/m) / 2^32), exact for t < 2^20 and
-// m <= 256 (the rounding error of the magic multiplier, below 2^-12, stays
-// under 1/m), is the high word of s * magic + h * magic, and
-// s - q m = (v + h) mod m - h is the residue of v in [-h, h]. Every constant
-// folds: two DP4As, one wide multiply-add, one IMAD.
+// The dot products start from the bit pattern of the float `base` (a multiple
+// of 256 m just above 1.5 * 2^23), so their sum is the bit pattern of
+// F = base + s. Then, in FP32,
+//   q = rint(F * inv_m)  (one FMA onto 1.5 * 2^23 rounds to an integer),
+//   F - (q - base/m) m   = base + r, exact,
+// whose low mantissa byte is r. q may be one off from the nearest quotient
+// (F < 2^24 and inv_m is within 2^-24 relative), so |r| <= m/2 + 1 <= 127 for
+// m <= 253: a residue of v all the same, and the sums of products that use it
+// are exact. For m = 255 the quotient is taken exactly in integers: with
+// t = s + h < 2^20, floor(t / m) = floor(t ceil(2^32/m) / 2^32).
+// The integer form for every modulus spends a wide multiply-add and an IMAD
+// after the dot products, all on the half-rate multiply pipe; in FP32 two
+// values share each instruction (residue_s2). Together with the order of the
+// stores (slice_rc_body) the slices of both operands fell from 67 to 54 us at
+// FP64 2048^3, from 133 to 101 for complex128 2401 x 1639 x 1203.
 template <int L> __device__ __forceinline__ int32_t residue_s(const Digits &x) {
     using C = Mod<L>;
     if constexpr (C::m == 256) {
         return int32_t(x.lo);
-    } else {
+    } else if constexpr (C::m == 255) {
         const uint32_t s = __dp4a(x.hi, C::whi, __dp4a(x.lo, C::wlo, C::cb));
         const uint32_t q = uint32_t((uint64_t(s) * C::magic + C::hmagic) >> 32);
         return int32_t(s - q * C::m);
+    } else {
+        const float F = __uint_as_float(__dp4a(x.hi, C::whi, __dp4a(x.lo, C::wlo, C::fbits)));
+        const float q = __fmaf_rn(F, 1.0f / float(C::m), 12582912.0f) - (12582912.0f + float(C::base_q));
+        return __float_as_int(__fmaf_rn(q, -float(C::m), F));
+    }
+}
+
+// The same for two values, the FP32 steps on both at once.
+template <int L> __device__ __forceinline__ void residue_s2(const Digits &x, const Digits &y, int32_t &a, int32_t &b) {
+    using C = Mod<L>;
+    if constexpr (C::m >= 255) {
+        a = residue_s<L>(x);
+        b = residue_s<L>(y);
+    } else {
+        const float inv = 1.0f / float(C::m), m = -float(C::m), off = -(12582912.0f + float(C::base_q));
+        const uint32_t fx = __dp4a(x.hi, C::whi, __dp4a(x.lo, C::wlo, C::fbits));
+        const uint32_t fy = __dp4a(y.hi, C::whi, __dp4a(y.lo, C::wlo, C::fbits));
+        asm("{\n.reg .b64 f, i, c, o, n, q;\n"
+            "mov.b64 f, {%2, %3};\nmov.b64 i, {%4, %4};\nmov.b64 c, {%5, %5};\nmov.b64 o, {%6, %6};\n"
+            "mov.b64 n, {%7, %7};\n"
+            "fma.rn.f32x2 q, f, i, c;\nadd.rn.f32x2 q, q, o;\nfma.rn.f32x2 q, q, n, f;\nmov.b64 {%0, %1}, q;\n}"
+            : "=r"(a), "=r"(b)
+            : "r"(fx), "r"(fy), "f"(inv), "f"(12582912.0f), "f"(off), "f"(m));
     }
 }
 
@@ -391,9 +428,12 @@ struct SliceOut {
 template <int L> __device__ __forceinline__ uint4 pack16(const Digits (&x)[16]) {
     uint32_t w[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
-        w[q] = pack_bytes(residue_s<L>(x[4 * q]), residue_s<L>(x[4 * q + 1]), residue_s<L>(x[4 * q + 2]),
-                          residue_s<L>(x[4 * q + 3]));
+    for (int q = 0; q < 4; ++q) {
+        int32_t r[4];
+        residue_s2<L>(x[4 * q], x[4 * q + 1], r[0], r[1]);
+        residue_s2<L>(x[4 * q + 2], x[4 * q + 3], r[2], r[3]);
+        w[q] = pack_bytes(r[0], r[1], r[2], r[3]);
+    }
     return make_uint4(w[0], w[1], w[2], w[3]);
 }
 __device__ __forceinline__ uint4 neg16(uint4 a) {  // residue of -x, byte-wise
@@ -483,19 +523,27 @@ __device__ __forceinline__ void slice_kc_body(const View &v, const RowStats &st,
 // row-contiguous source: a 64-row x KT-k tile is read along rows, scaled,
 // and its integers are transposed once through shared memory; then a thread
 // owns 16 consecutive k of one row and one component, as in the
-// k-contiguous kernel (complex: warps 0-3 the real parts, 4-7 the imaginary).
+// k-contiguous kernel (complex: warps 0-3 the real parts, 4-7 the imaginary),
+// adjacent threads the next 16 k of that row: a warp's stores are whole
+// 64-byte (complex: 32-byte) pieces of rows. Stores of 16 bytes to 32 rows
+// instead, conflict-free to read from a plain transposed tile, run at 1.5 to
+// 2.6 TB/s against 5.7 to 6.3 for 64-byte pieces. So column k of the tile is
+// shifted by 4 (k / 16), which makes this order of reads conflict-free too.
 // grid (Kc/KT, Rp/64), block 256; smem holds slice_rc_smem_bytes<ROLE>()
 // bytes (the transposed tile, then the 64 row exponents).
+constexpr int kRcLd = 64 + 12;  // row of the transposed tile, in int64
+__device__ __forceinline__ int rc_at(int k, int r) { return k * kRcLd + r + (k >> 4) * 4; }
 template <int ROLE> constexpr size_t slice_rc_smem_bytes() {
-    return size_t(ROLE ? 2 : 1) * (ROLE ? 32 : 64) * (64 + 1) * sizeof(int64_t) + 64 * sizeof(int);
+    return size_t(ROLE ? 2 : 1) * (ROLE ? 32 : 64) * kRcLd * sizeof(int64_t) + 64 * sizeof(int);
 }
 template <typename T, int ROLE>
 __device__ __forceinline__ void slice_rc_body(const View &v, const RowStats &st, const Decision *dec, int *expo,
                                               const SliceOut &o, int64_t bx, int64_t by, int tid, void *smem) {
     constexpr int KT = ROLE ? 32 : 64;
     constexpr int CPL = ROLE ? 2 : 1;
-    int64_t (*tile)[KT][64 + 1] = reinterpret_cast<int64_t (*)[KT][64 + 1]>(smem);
-    int *s_e = reinterpret_cast<int *>(static_cast<char *>(smem) + size_t(CPL) * KT * (64 + 1) * sizeof(int64_t));
+    constexpr int COMP = KT * kRcLd;  // one component's tile
+    int64_t *tile = static_cast<int64_t *>(smem);
+    int *s_e = reinterpret_cast<int *>(tile + CPL * COMP);
     const int nmod = dec->nmod;
     if (nmod == 0) return;
     const int Q = dec->q;
@@ -527,8 +575,8 @@ __device__ __forceinline__ void slice_rc_body(const View &v, const RowStats &st,
                     if (r + 1 < v.R) x = __ldcg(reinterpret_cast<const double2 *>(q));
                     else if (r < v.R) x.x = q[0];
                 }
-                tile[0][kk][tr] = scale_round(x.x, e0);
-                tile[0][kk][tr + 1] = scale_round(x.y, e1);
+                *reinterpret_cast<longlong2 *>(&tile[rc_at(kk, tr)]) =
+                    make_longlong2(scale_round(x.x, e0), scale_round(x.y, e1));
             }
         }
     }
@@ -541,19 +589,18 @@ __device__ __forceinline__ void slice_rc_body(const View &v, const RowStats &st,
             const int kk = tk + 4 * i;
             double re = 0, im = 0;
             if (r < v.R && k0 + kk < v.K) load_elem<T>(v, r, k0 + kk, false, re, im);
-            tile[0][kk][tr] = scale_round(re, e);
-            if (ROLE) tile[CPL - 1][kk][tr] = scale_round(im, e);
+            tile[rc_at(kk, tr)] = scale_round(re, e);
+            if (ROLE) tile[(CPL - 1) * COMP + rc_at(kk, tr)] = scale_round(im, e);
         }
     }
     __syncthreads();
     constexpr int TPR = KT / 16;  // threads per row and component
     static_assert(64 * TPR * CPL == 256, "one 16-k word per thread");
-    // a warp reads 32 consecutive rows of one k-group: conflict-free
     const int comp = tid / (64 * TPR), idx = tid % (64 * TPR);
-    const int wr = idx % 64, wk = (idx / 64) * 16;
+    const int wr = idx / TPR, wk = idx % TPR * 16;
     Digits d[16];
 #pragma unroll
-    for (int q = 0; q < 16; ++q) d[q] = digits_of(tile[comp][wk + q][wr]);
+    for (int q = 0; q < 16; ++q) d[q] = digits_of(tile[comp * COMP + rc_at(wk + q, wr)]);
     if (comp == 0) store_all<ROLE, 0>(o, nmod, r0 + wr, k0 + wk, d);
     else if (ROLE) store_all<ROLE, 1>(o, nmod, r0 + wr, k0 + wk, d);
 }
