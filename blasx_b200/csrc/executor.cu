@@ -310,7 +310,8 @@ __device__ __forceinline__ void emulated_task(const ReqDesc &d, const Task &t, i
             // two 128-thread blocks at a time
             const int half = tid >> 7, ht = tid & 127;
             for (int64_t b = t.first + half; b < t.first + t.count; b += 2)
-                oz::reconstruct_body<T, CPLX>(d.ra, d.dec, b % d.recon_gx, b / d.recon_gx, ht);
+                oz::reconstruct_body<T, CPLX>(d.ra, d.dec, b % d.recon_gx, b / d.recon_gx, ht,
+                                              reinterpret_cast<double *>(work) + half * 4 * oz::kReconShared<CPLX>);
             break;
         }
         default:

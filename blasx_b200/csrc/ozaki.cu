@@ -68,7 +68,8 @@ __global__ void __launch_bounds__(256, 4) slice_both_kernel(SliceSide a, SliceSi
 
 template <typename T, bool CPLX>
 __global__ void __launch_bounds__(128) reconstruct_kernel(const ReconArgs a, const Decision *dec) {
-    reconstruct_body<T, CPLX>(a, dec, blockIdx.x, blockIdx.y, threadIdx.x);
+    __shared__ __align__(16) double sh[4 * kReconShared<CPLX>];
+    reconstruct_body<T, CPLX>(a, dec, blockIdx.x, blockIdx.y, threadIdx.x, sh);
 }
 
 std::once_flag g_tables_once;

@@ -818,153 +818,188 @@ __device__ __forceinline__ bool recon_keep(const ReconArgs &a, int64_t i, int64_
     return a.uplo == 0 || (a.uplo == 1 ? i - j <= a.diag : i - j >= a.diag);
 }
 
-template <typename T, int N>
-__device__ __forceinline__ void recon_real(const ReconArgs &a, int64_t i0, int64_t j) {
-    uint32_t w[N];
-    gather4<N>(a.U, a.Jp * a.Ip, j * a.Ip + i0, w);
+// Whether a warp's 128 rows from w0 of column j lie inside C and the triangle
+// as a whole, and whether any of them does.
+__device__ __forceinline__ bool recon_whole(const ReconArgs &a, int64_t w0, int64_t j) {
+    return w0 + 127 < a.M && (a.uplo == 0 || (a.uplo == 1 ? w0 + 127 - j <= a.diag : w0 - j >= a.diag));
+}
+__device__ __forceinline__ bool recon_any(const ReconArgs &a, int64_t w0, int64_t j) {
+    const int64_t last = min(w0 + 127, a.M - 1);
+    return a.uplo == 0 || (a.uplo == 1 ? w0 - j <= a.diag : last - j >= a.diag);
+}
+// Minus the exponents of rows i0 .. i0 + 3 and column j (i0 a multiple of 4).
+__device__ __forceinline__ void recon_scales(const ReconArgs &a, int64_t i0, int64_t j, int (&sc)[4]) {
     const int fj = a.fb[j];
-    T *C = static_cast<T *>(a.C);
-    auto put = [&](int64_t i, double val) {
-        T *cp = C + i + j * a.ldc;
-        double r = a.ar * val;
-        if (!a.beta_zero) r = fma(a.br, double(*cp), r);
-        *cp = T(r);
-    };
+    if (i0 + 3 < a.M) {
+        const int4 e = *reinterpret_cast<const int4 *>(a.ea + i0);
+        sc[0] = -(e.x + fj);
+        sc[1] = -(e.y + fj);
+        sc[2] = -(e.z + fj);
+        sc[3] = -(e.w + fj);
+    } else {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) sc[q] = i0 + q < a.M ? -(a.ea[i0 + q] + fj) : 0;
+    }
+}
+// The CRT values of 4 rows of one column (w: their residues).
+template <int N>
+__device__ __forceinline__ void recon_values(const uint32_t (&w)[N], const int (&sc)[4], double (&x)[4]) {
     if constexpr (N <= kMaxFpCrt) {
         double S[4][fp_limbs<N>()];
         crt_sums4<N>(w, S);
-        T *cp = C + i0 + j * a.ldc;
-        if (a.uplo == 0 && i0 + 3 < a.M && (reinterpret_cast<uintptr_t>(cp) & 15) == 0) {
-            // 4 whole rows, 16-byte aligned: vector loads and stores of C and
-            // the row exponents, the same arithmetic per entry as put
-            const int4 e = *reinterpret_cast<const int4 *>(a.ea + i0);
-            double r[4] = {crt_round<N>(S[0], -(e.x + fj)), crt_round<N>(S[1], -(e.y + fj)),
-                           crt_round<N>(S[2], -(e.z + fj)), crt_round<N>(S[3], -(e.w + fj))};
 #pragma unroll
-            for (int q = 0; q < 4; ++q) r[q] = a.ar * r[q];
-            if constexpr (std::is_same<T, double>::value) {
-                double2 *v = reinterpret_cast<double2 *>(cp);
-                if (!a.beta_zero) {
-                    const double2 c0 = v[0], c1 = v[1];
-                    r[0] = fma(a.br, c0.x, r[0]);
-                    r[1] = fma(a.br, c0.y, r[1]);
-                    r[2] = fma(a.br, c1.x, r[2]);
-                    r[3] = fma(a.br, c1.y, r[3]);
-                }
-                v[0] = make_double2(r[0], r[1]);
-                v[1] = make_double2(r[2], r[3]);
-            } else {
-                float4 *v = reinterpret_cast<float4 *>(cp);
-                if (!a.beta_zero) {
-                    const float4 c = *v;
-                    r[0] = fma(a.br, double(c.x), r[0]);
-                    r[1] = fma(a.br, double(c.y), r[1]);
-                    r[2] = fma(a.br, double(c.z), r[2]);
-                    r[3] = fma(a.br, double(c.w), r[3]);
-                }
-                *v = make_float4(float(r[0]), float(r[1]), float(r[2]), float(r[3]));
-            }
-            return;
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int64_t i = i0 + q;
-            if (i < a.M && recon_keep(a, i, j)) put(i, crt_round<N>(S[q], -(a.ea[i] + fj)));
-        }
+        for (int q = 0; q < 4; ++q) x[q] = crt_round<N>(S[q], sc[q]);
     } else {
+        // (selects, so that x stays in registers)
 #pragma unroll 1
         for (int q = 0; q < 4; ++q) {
-            const int64_t i = i0 + q;
-            if (i >= a.M) break;
-            if (!recon_keep(a, i, j)) continue;
-            put(i, crt_to_double<N>(w, q, -(a.ea[i] + fj)));
+            const double v = crt_to_double<N>(w, q, q < 2 ? (q ? sc[1] : sc[0]) : (q == 2 ? sc[2] : sc[3]));
+#pragma unroll
+            for (int p = 0; p < 4; ++p)
+                if (p == q) x[p] = v;
         }
     }
 }
 
+// Rows w0 .. w0 + 127 of column j, by one warp; lane l computes rows 4 l to
+// 4 l + 3, whose residues are one word per modulus. Where a column of C is
+// not 16-byte aligned (odd ldc), crosses the triangle or ends, the warp hands
+// its values over through sh (128 doubles) so that lane l updates rows l, l +
+// 32, ...: whole lines of C instead of one entry in four per access (FP32
+// 3001 x 1777: RECON_FIGURES).
 template <typename T, int N>
-__device__ __forceinline__ void recon_cplx(const ReconArgs &a, int64_t i0, int64_t j) {
+__device__ __forceinline__ void recon_real(const ReconArgs &a, int64_t w0, int64_t j, int lane, double *sh) {
+    const int64_t i0 = w0 + 4 * lane;
+    uint32_t w[N];
+    gather4<N>(a.U, a.Jp * a.Ip, j * a.Ip + i0, w);
+    int sc[4];
+    recon_scales(a, i0, j, sc);
+    double r[4];
+    recon_values<N>(w, sc, r);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) r[q] = a.ar * r[q];
+    T *C = static_cast<T *>(a.C) + j * a.ldc;
+    if (recon_whole(a, w0, j) && (reinterpret_cast<uintptr_t>(C) & 15) == 0) {
+        T *cp = C + i0;
+        if constexpr (std::is_same<T, double>::value) {
+            double2 *v = reinterpret_cast<double2 *>(cp);
+            if (!a.beta_zero) {
+                const double2 c0 = v[0], c1 = v[1];
+                r[0] = fma(a.br, c0.x, r[0]);
+                r[1] = fma(a.br, c0.y, r[1]);
+                r[2] = fma(a.br, c1.x, r[2]);
+                r[3] = fma(a.br, c1.y, r[3]);
+            }
+            v[0] = make_double2(r[0], r[1]);
+            v[1] = make_double2(r[2], r[3]);
+        } else {
+            float4 *v = reinterpret_cast<float4 *>(cp);
+            if (!a.beta_zero) {
+                const float4 c = *v;
+                r[0] = fma(a.br, double(c.x), r[0]);
+                r[1] = fma(a.br, double(c.y), r[1]);
+                r[2] = fma(a.br, double(c.z), r[2]);
+                r[3] = fma(a.br, double(c.w), r[3]);
+            }
+            *v = make_float4(float(r[0]), float(r[1]), float(r[2]), float(r[3]));
+        }
+        return;
+    }
+    __syncwarp();  // the warp has left sh of an earlier column
+    reinterpret_cast<double2 *>(sh)[2 * lane] = make_double2(r[0], r[1]);
+    reinterpret_cast<double2 *>(sh)[2 * lane + 1] = make_double2(r[2], r[3]);
+    __syncwarp();
+    T cin[4];
+    bool keep[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int64_t i = w0 + lane + 32 * q;
+        keep[q] = i < a.M && recon_keep(a, i, j);
+        cin[q] = keep[q] && !a.beta_zero ? C[i] : T(0);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        double v = sh[lane + 32 * q];
+        if (!a.beta_zero) v = fma(a.br, double(cin[q]), v);
+        if (keep[q]) C[w0 + lane + 32 * q] = T(v);
+    }
+}
+
+// The same for complex C, always by way of sh (256 doubles): an entry is 16
+// (8) bytes, of which 32 adjacent ones make whole lines.
+template <typename T, int N>
+__device__ __forceinline__ void recon_cplx(const ReconArgs &a, int64_t w0, int64_t j, int lane, double *sh) {
     using R = typename Elem<T>::R;
+    const int64_t i0 = w0 + 4 * lane;
     const int64_t plane = 2 * a.Jp * a.Ip;
-    uint32_t wr[N], wi[N];
-    gather4<N>(a.U, plane, j * a.Ip + i0, wr);
-    gather4<N>(a.U, plane, (a.Jp + j) * a.Ip + i0, wi);
-    const int fj = a.fb[j];
-    R *C = static_cast<R *>(a.C);
-    // one entry: (re, im) loaded and stored as one vector (16 bytes for
-    // complex128, 8 for complex64) when C is aligned to that size
+    int sc[4];
+    recon_scales(a, i0, j, sc);
+    __syncwarp();  // the warp has left sh of an earlier column
+#pragma unroll
+    for (int part = 0; part < 2; ++part) {  // the real parts, then the imaginary
+        uint32_t w[N];
+        gather4<N>(a.U, plane, (j + (part ? a.Jp : 0)) * a.Ip + i0, w);
+        double x[4];
+        recon_values<N>(w, sc, x);
+        double2 *d = reinterpret_cast<double2 *>(sh + 128 * part);
+        d[2 * lane] = make_double2(x[0], x[1]);
+        d[2 * lane + 1] = make_double2(x[2], x[3]);
+    }
+    __syncwarp();
+    R *C = static_cast<R *>(a.C) + 2 * j * a.ldc;
+    // one entry as one vector (16 bytes for complex128, 8 for complex64) when
+    // C is aligned to that size
     using V = typename std::conditional<std::is_same<R, double>::value, double2, float2>::type;
     const bool vec = (reinterpret_cast<uintptr_t>(a.C) & (sizeof(V) - 1)) == 0;
-    auto put = [&](int64_t i, double xr, double xi) {
-        R *cp = C + 2 * (i + j * a.ldc);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int64_t i = w0 + lane + 32 * q;
+        if (i >= a.M || !recon_keep(a, i, j)) continue;
+        const double xr = sh[lane + 32 * q], xi = sh[128 + lane + 32 * q];
+        R *cp = C + 2 * i;
         double vr = a.ar * xr - a.ai * xi, vi = a.ar * xi + a.ai * xr;
+        V c;
+        c.x = c.y = R(0);
+        if (!a.beta_zero) {
+            if (vec) {
+                c = *reinterpret_cast<const V *>(cp);
+            } else {
+                c.x = cp[0];
+                c.y = cp[1];
+            }
+            const double cr = double(c.x), ci = double(c.y);
+            vr += a.br * cr - a.bi * ci;
+            vi += a.br * ci + a.bi * cr;
+        }
         if (vec) {
-            V *vp = reinterpret_cast<V *>(cp);
-            if (!a.beta_zero) {
-                const V c = *vp;
-                const double cr = double(c.x), ci = double(c.y);
-                vr += a.br * cr - a.bi * ci;
-                vi += a.br * ci + a.bi * cr;
-            }
-            V o;
-            o.x = R(vr);
-            o.y = R(vi);
-            *vp = o;
+            c.x = R(vr);
+            c.y = R(vi);
+            *reinterpret_cast<V *>(cp) = c;
         } else {
-            if (!a.beta_zero) {
-                const double cr = double(cp[0]), ci = double(cp[1]);
-                vr += a.br * cr - a.bi * ci;
-                vi += a.br * ci + a.bi * cr;
-            }
             cp[0] = R(vr);
             cp[1] = R(vi);
         }
-    };
-    if constexpr (N <= kMaxFpCrt) {
-        // the real parts of the 4 rows, then the imaginary parts
-        double xr[4], S[4][fp_limbs<N>()];
-        int sc[4];
-        bool live[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int64_t i = i0 + q;
-            live[q] = i < a.M && recon_keep(a, i, j);
-            sc[q] = live[q] ? -(a.ea[i] + fj) : 0;
-        }
-        crt_sums4<N>(wr, S);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) xr[q] = crt_round<N>(S[q], sc[q]);
-        crt_sums4<N>(wi, S);
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-            if (live[q]) put(i0 + q, xr[q], crt_round<N>(S[q], sc[q]));
-    } else {
-#pragma unroll 1
-        for (int q = 0; q < 4; ++q) {
-            const int64_t i = i0 + q;
-            if (i >= a.M) break;
-            if (!recon_keep(a, i, j)) continue;
-            const int sc = -(a.ea[i] + fj);
-            put(i, crt_to_double<N>(wr, q, sc), crt_to_double<N>(wi, q, sc));
-        }
     }
 }
 
-// One thread per 4 consecutive rows i of a column j. The modulus count is
-// read on the device; the switch is uniform, each case fully unrolled.
-// Block (bx, by) of 128 threads: column j0 + by, rows 512 bx .. 512 bx + 511.
+// The modulus count is read on the device; the switch is uniform, each case
+// fully unrolled. Block (bx, by) of 128 threads: column j0 + by, rows 512 bx
+// .. 512 bx + 511, 128 per warp; a warp without an entry to write does
+// nothing. sh: kReconShared<CPLX> doubles for each warp of the block.
+template <bool CPLX> constexpr int kReconShared = CPLX ? 256 : 128;
 template <typename T, bool CPLX>
 __device__ __forceinline__ void reconstruct_body(const ReconArgs &a, const Decision *dec, int64_t bx, int64_t by,
-                                                 int tid) {
+                                                 int tid, double *sh) {
     const int n = dec->nmod;
     if (n == 0) return;
     const int64_t j = a.j0 + by;
-    const int64_t i0 = (bx * 128 + tid) * 4;
-    if (i0 >= a.M || j >= a.N) return;
-#define BX_RECON_CASE(NN)                                     \
-    case NN:                                                  \
-        if constexpr (CPLX) recon_cplx<T, NN>(a, i0, j);      \
-        else recon_real<T, NN>(a, i0, j);                     \
+    const int64_t w0 = bx * 512 + (tid >> 5) * 128;
+    if (w0 >= a.M || j >= a.N || !recon_any(a, w0, j)) return;
+    sh += (tid >> 5) * kReconShared<CPLX>;
+#define BX_RECON_CASE(NN)                                                  \
+    case NN:                                                               \
+        if constexpr (CPLX) recon_cplx<T, NN>(a, w0, j, tid & 31, sh);     \
+        else recon_real<T, NN>(a, w0, j, tid & 31, sh);                    \
         break;
     switch (n) {
         BX_RECON_CASE(6) BX_RECON_CASE(7) BX_RECON_CASE(8) BX_RECON_CASE(9) BX_RECON_CASE(10)
