@@ -152,8 +152,8 @@ struct Context {
     cudaStream_t h2d = nullptr;      // host -> device copies
     cudaStream_t d2h = nullptr;      // device -> host copies
     std::mutex host_mu;              // serialises host-pipeline calls
-    // pinned host slots the emulated path copies its device decision and
-    // error flag into (valid once the stream has passed the copy)
+    // pinned, mapped host slots the emulated path's reconstruction writes its
+    // decision and error flag to (valid once the stream has passed the call)
     void *last_decision = nullptr;   // oz::Decision
     int *last_error_flag = nullptr;
 };
