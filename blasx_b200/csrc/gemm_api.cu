@@ -100,6 +100,7 @@ int device_entry(DType dt, int ta, int tb, int M, int N, int K, cplx alpha, cons
     // NULL is the CUDA legacy default stream, as everywhere in the CUDA API
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (g.alpha_zero() || g.K == 0) return launch_scale(g, s);
+    g.resident = true;
     return device_gemm(g, s);
 }
 

@@ -302,13 +302,18 @@ int ozaki_run(const Gemm &g, cudaStream_t s, int mode, void *ws, int num_sms, vo
     return BLASX_OK;
 }
 
-template <typename T> int ozaki_t(const Gemm &g, cudaStream_t s, int mode) {
+template <typename T> int ozaki_t(const Gemm &g, cudaStream_t s, int mode, bool optional) {
     Context *ctx = context();
     if (!ctx) return last_status();
     BX_TRY(oz::upload_crt_tables());
     const oz::Plan pl = oz::make_plan(g);
     void *ws = nullptr;
-    BX_CUDA(dev_malloc_async(&ws, pl.bytes, s));
+    const cudaError_t got = dev_malloc_async(&ws, pl.bytes, s);
+    if (got == cudaErrorMemoryAllocation && optional) {
+        cudaGetLastError();
+        return kNoScratch;
+    }
+    BX_CUDA(got);
     struct Free {
         void *p;
         cudaStream_t s;
@@ -319,12 +324,12 @@ template <typename T> int ozaki_t(const Gemm &g, cudaStream_t s, int mode) {
 
 }  // namespace
 
-int ozaki_gemm(const Gemm &g, cudaStream_t s, int mode) {
+int ozaki_gemm(const Gemm &g, cudaStream_t s, int mode, bool optional) {
     switch (g.dt) {
-        case DType::F64: return ozaki_t<double>(g, s, mode);
-        case DType::F32: return ozaki_t<float>(g, s, mode);
-        case DType::C64: return ozaki_t<oz::cpair>(g, s, mode);
-        default: return ozaki_t<oz::zpair>(g, s, mode);
+        case DType::F64: return ozaki_t<double>(g, s, mode, optional);
+        case DType::F32: return ozaki_t<float>(g, s, mode, optional);
+        case DType::C64: return ozaki_t<oz::cpair>(g, s, mode, optional);
+        default: return ozaki_t<oz::zpair>(g, s, mode, optional);
     }
 }
 

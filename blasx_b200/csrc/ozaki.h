@@ -94,15 +94,17 @@ extern const int kModuli[kMaxModuli];
 // Whether precision mode `mode` runs g on the emulated path. Mode 2 (ozaki)
 // always does when K is within the exact range; mode 1 (native) never; mode
 // 0 (auto) where the emulated path measured faster than the native kernels
-// on one B200 (device-resident n^3 sweep, 256 <= n <= 4096): FP64 from
-// about 1800^3, FP32 from about 640^3, complex128 from about 1200^3. Small K
-// also loses: reconstruction costs about as much per C entry as ~350 native
-// FP64 multiply-adds, whatever K is.
+// on one B200 (dispatch.cu has the lines and the figures). Small K also loses:
+// reconstruction costs about as much per C entry as a few hundred native FP64
+// multiply-adds, whatever K is.
 bool ozaki_selected(const Gemm &g, int mode);
 
 // Emulated GEMM on device-resident operands. Chooses the modulus count on
 // the device; falls back to the native kernel on the device when needed.
-int ozaki_gemm(const Gemm &g, cudaStream_t s, int mode);
+// With `optional`, a scratch that cannot be allocated gives kNoScratch, with
+// nothing launched and no error recorded.
+constexpr int kNoScratch = -1;
+int ozaki_gemm(const Gemm &g, cudaStream_t s, int mode, bool optional = false);
 
 // Scratch bytes the emulated pipeline needs for g, and the pipeline itself
 // on a caller-provided scratch of at least that size (allocates nothing;

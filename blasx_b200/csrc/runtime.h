@@ -75,6 +75,10 @@ struct Gemm {
     // entries (row == col, shifted by diag like uplo) are set to zero once
     // the product is complete.
     bool herm_out = false;
+    // A call on device-resident operands: emulated scratch comes from the
+    // device's memory pool, outside any HBM budget, and the native kernels
+    // stand in when there is none (ozaki_selected).
+    bool resident = false;
 
     bool alpha_zero() const { return alpha.re == 0 && alpha.im == 0; }
     bool beta_zero() const { return beta.re == 0 && beta.im == 0; }
@@ -108,6 +112,7 @@ struct Trsm {
     int64_t lda;
     void *B;
     int64_t ldb;
+    bool resident = false;  // as Gemm::resident, for the updates
     int64_t order() const { return left ? M : N; }
 };
 

@@ -236,6 +236,7 @@ int tri_device_entry(bool mult, DType dt, int side, int uplo, int trans, int dia
     t.alpha = alpha;
     t.A = A; t.lda = lda;
     t.B = B; t.ldb = ldb;
+    t.resident = true;
     bool emulated = false;
     if (!mult) return trsm_device(t, s, &emulated);
     TrmmScratch w = trmm_scratch_sizes(t);

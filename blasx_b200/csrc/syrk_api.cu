@@ -216,8 +216,9 @@ int syrk_device(DType dt, int uplo, int trans, int N, int K, cplx alpha, const v
     if (N == 0) return BLASX_OK;
     Context *c = context();
     if (!c) return last_status();
-    const Gemm g = tri_gemm(dt, CblasColMajor, uplo, trans, N, K, alpha, A, lda, A, lda, beta, C, ldc);
+    Gemm g = tri_gemm(dt, CblasColMajor, uplo, trans, N, K, alpha, A, lda, A, lda, beta, C, ldc);
     if (g.alpha_zero() || g.K == 0) return launch_scale(g, s);
+    g.resident = true;
     return device_gemm(g, s);
 }
 

@@ -289,6 +289,7 @@ Gemm update_gemm(const Trsm &t, Range tgt, Range src, cplx alpha, cplx beta) {
     g.alpha = alpha;
     g.beta = beta;
     g.K = src.size();
+    g.resident = t.resident;
     if (t.left) {
         g.M = tgt.size();
         g.N = t.N;
