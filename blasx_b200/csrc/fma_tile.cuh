@@ -233,25 +233,38 @@ __device__ __forceinline__ void fma_tile(const FmaParams<T> &fp, int tile, T *sm
     } else {
         __syncthreads();
     }
-    for (int e = tid; e < (c_hi - c_lo) * BM; e += TL::THREADS) {
-        const int r = e % BM, c = c_lo + e / BM;
-        const int gm = m0 + r, gn = n0 + c;
-        if (gm >= p.M || gn >= p.N) continue;
-        if (p.uplo && (p.uplo == 1 ? gm - int64_t(gn) > p.diag : gm - int64_t(gn) < p.diag)) continue;
-        T v = Ar::zero();
-        if constexpr (SPLIT) {
-            for (int q = 0; q < splits; ++q)
+    // four entries at a time, their C values loaded before any is stored
+    constexpr int BATCH = 4;
+    const int entries = (c_hi - c_lo) * BM;
+    for (int e0 = tid; e0 < entries; e0 += BATCH * TL::THREADS) {
+        T cin[BATCH];
+        bool in[BATCH];
 #pragma unroll
-                for (int g = 0; g < TL::KS; ++g)
-                    v = Ar::add(v, fma_cluster_read(&smem[g * PART + c * LD + r], uint32_t(q)));
-        } else {
-#pragma unroll
-            for (int g = 0; g < TL::KS; ++g) v = Ar::add(v, smem[g * PART + c * LD + r]);
+        for (int b = 0; b < BATCH; ++b) {
+            const int e = e0 + b * TL::THREADS;
+            const int gm = m0 + e % BM, gn = n0 + c_lo + e / BM;
+            in[b] = e < entries && gm < p.M && gn < p.N &&
+                    !(p.uplo && (p.uplo == 1 ? gm - int64_t(gn) > p.diag : gm - int64_t(gn) < p.diag));
+            cin[b] = in[b] && !p.beta_zero ? p.C[gm + gn * p.ldc] : Ar::zero();
         }
-        T *cp = &p.C[gm + gn * p.ldc];
-        v = Ar::mul(p.alpha, v);
-        if (!p.beta_zero) v = Ar::add(v, Ar::mul(p.beta, *cp));
-        *cp = v;
+#pragma unroll
+        for (int b = 0; b < BATCH; ++b) {
+            if (!in[b]) continue;
+            const int e = e0 + b * TL::THREADS, r = e % BM, c = c_lo + e / BM;
+            T v = Ar::zero();
+            if constexpr (SPLIT) {
+                for (int q = 0; q < splits; ++q)
+#pragma unroll
+                    for (int g = 0; g < TL::KS; ++g)
+                        v = Ar::add(v, fma_cluster_read(&smem[g * PART + c * LD + r], uint32_t(q)));
+            } else {
+#pragma unroll
+                for (int g = 0; g < TL::KS; ++g) v = Ar::add(v, smem[g * PART + c * LD + r]);
+            }
+            v = Ar::mul(p.alpha, v);
+            if (!p.beta_zero) v = Ar::add(v, Ar::mul(p.beta, cin[b]));
+            p.C[m0 + r + (n0 + c) * p.ldc] = v;
+        }
     }
     if constexpr (SPLIT) dmma_cluster_sync();  // no CTA leaves while another reads its partial tiles
 }

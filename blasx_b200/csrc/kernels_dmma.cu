@@ -22,19 +22,25 @@ namespace {
 
 using namespace dev;
 
-// One CTA per tile; or, for the emulated path's fallback, one resident set of
-// CTAs that take tiles from a counter: it usually has nothing to do, and the
-// exits of a CTA per tile took 6 us at 2048^3. (Tiles dealt out in advance
-// instead took 6% longer when 4096 x 3000 x 2500 did fall back.)
 template <bool CPLX, bool AKC, bool BKC, int KI, int G>
 __global__ void __launch_bounds__(Tile<CPLX, G>::THREADS, Tile<CPLX, G>::PER_SM)
     dmma_gemm_kernel(const DmmaParams p) {
     if (p.guard && *p.guard != 0) return;  // the emulated path produced C
     extern __shared__ __align__(16) double smem[];
-    if (!p.queue) {
-        dmma_tile<CPLX, AKC, BKC, KI, G>(p, blockIdx.x, smem);
-        return;
-    }
+    dmma_tile<CPLX, AKC, BKC, KI, G>(p, blockIdx.x, smem);
+}
+
+// The emulated path's fallback: one resident set of CTAs that take tiles from
+// a counter. It usually has nothing to do, and the exits of a CTA per tile took
+// 6 us at 2048^3. (From four sets of tiles on it is a CTA per tile again: the
+// counter costs a product that does fall back 2.6%, 4096 x 3000 x 2500, tiles
+// dealt out in advance 6%, and the exits cost a large product less. A kernel
+// of its own: the loop in the plain one made that 3% slower.)
+template <bool CPLX, bool AKC, bool BKC, int KI, int G>
+__global__ void __launch_bounds__(Tile<CPLX, G>::THREADS, Tile<CPLX, G>::PER_SM)
+    dmma_queue_kernel(const DmmaParams p) {
+    if (*p.guard != 0) return;
+    extern __shared__ __align__(16) double smem[];
     __shared__ int s_tile;
     const int tiles = p.tiles_m * p.tiles_n;
     for (;;) {
@@ -97,8 +103,15 @@ int launch_cfg(const DmmaParams &p, int splits, cudaStream_t s) {
         }
     }
     auto kern = dmma_gemm_kernel<CPLX, AKC, BKC, KI, G>;
+    int64_t grid = tiles;
+    if constexpr (G != 0 && (CPLX || KI == 16)) {
+        const int64_t set = int64_t(TL::PER_SM) * num_sms();
+        if (p.guard && p.queue && tiles <= 4 * set) {
+            kern = dmma_queue_kernel<CPLX, AKC, BKC, KI, G>;
+            grid = std::min(tiles, set);
+        }
+    }
     BX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    const int64_t grid = p.queue ? std::min<int64_t>(tiles, int64_t(TL::PER_SM) * num_sms()) : tiles;
     kern<<<unsigned(grid), TL::THREADS, smem, s>>>(p);
     BX_CUDA(cudaGetLastError());
     count_launch();
@@ -138,7 +151,8 @@ struct TileModel {
 constexpr double kSplitCycles = 8000.0;
 constexpr TileModel kReal[] = {{1, 64, 64, 3, {0.55, 0.79, 0.87, 0}},
                                {3, 64, 48, 4, {0.53, 0.73, 0.77, 0.85}},
-                               {2, 32, 32, 4, {0.43, 0.61, 0.70, 0.774}}};
+                               {2, 32, 32, 4, {0.43, 0.61, 0.70, 0.72}},
+                               {0, 128, 128, 1, {0.78, 0, 0, 0}}};  // a single, nearly full wave
 constexpr TileModel kCplx[] = {{1, 64, 64, 2, {0.72, 0.86, 0, 0}}, {2, 32, 32, 4, {0.56, 0.76, 0.80, 0.83}}};
 
 template <int COUNT> Geometry pick_geometry(const TileModel (&models)[COUNT], double macs, const Gemm &g) {
@@ -152,7 +166,10 @@ template <int COUNT> Geometry pick_geometry(const TileModel (&models)[COUNT], do
         for (int s = 1; s == 1 || (s <= max_splits && g.K >= int64_t(32) * s && tiles < sms); s *= 2) {
             const int64_t ctas = tiles * s, round = sms * m.per_sm, rest = ctas % round;
             const int64_t n = (rest + sms - 1) / sms;
-            const double share = macs * m.bm * m.bn * double((g.K + s - 1) / s) / 64.0;  // one CTA, its pipe to itself
+            // one CTA, its pipe to itself; 32x32 tiles of two k-contiguous
+            // operands run 15% below the fraction of the other layouts
+            const double layout = m.g == 2 && macs == 1.0 && g.ta != NoTrans && g.tb == NoTrans ? 1.15 : 1.0;
+            const double share = layout * macs * m.bm * m.bn * double((g.K + s - 1) / s) / 64.0;
             const double t = share * (double(ctas / round) * m.per_sm / m.eff[m.per_sm - 1] +
                                       (n ? double(n) / m.eff[n - 1] : 0.0)) +
                              (s > 1 ? kSplitCycles : 0.0);

@@ -35,17 +35,20 @@ template <> struct Cfg<c2> {
     static constexpr int64_t min_k = 64;
 };
 
-// One CTA per tile, or (with a queue: the emulated path's fallback) a resident
-// set of CTAs that take tiles from the counter, as dmma_gemm_kernel.
 template <typename TL, typename T, bool AKC, bool BKC, int PER_SM>
-__global__ void __launch_bounds__(TL::THREADS, PER_SM)
-    fma_gemm_kernel(const FmaParams<T> p, const int *guard, int *queue) {
+__global__ void __launch_bounds__(TL::THREADS, PER_SM) fma_gemm_kernel(const FmaParams<T> p, const int *guard) {
     if (guard && *guard != 0) return;  // the emulated path produced C
     extern __shared__ __align__(16) unsigned char smem[];
-    if (!queue) {
-        fma_tile<TL, T, AKC, BKC, false>(p, blockIdx.x, reinterpret_cast<T *>(smem), 0, 1);
-        return;
-    }
+    fma_tile<TL, T, AKC, BKC, false>(p, blockIdx.x, reinterpret_cast<T *>(smem), 0, 1);
+}
+
+// The emulated path's fallback: a resident set of CTAs that take tiles from
+// the counter, as dmma_queue_kernel.
+template <typename TL, typename T, bool AKC, bool BKC, int PER_SM>
+__global__ void __launch_bounds__(TL::THREADS, PER_SM)
+    fma_queue_kernel(const FmaParams<T> p, const int *guard, int *queue) {
+    if (*guard != 0) return;
+    extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_tile;
     const int tiles = p.tiles_m * p.tiles_n;
     for (;;) {
@@ -115,10 +118,16 @@ int launch_tile(const Gemm &g, int splits, cudaStream_t s) {
             return BLASX_OK;
         }
     }
-    auto kern = fma_gemm_kernel<TL, T, AKC, BKC, PER_SM>;
-    BX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    const int64_t grid = g.queue ? std::min<int64_t>(tiles, int64_t(PER_SM) * kSms) : tiles;
-    kern<<<unsigned(grid), TL::THREADS, smem, s>>>(p, g.guard, g.queue);
+    const int64_t set = int64_t(PER_SM) * kSms;
+    if (g.guard && g.queue && tiles <= 4 * set) {
+        auto kern = fma_queue_kernel<TL, T, AKC, BKC, PER_SM>;
+        BX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        kern<<<unsigned(std::min(tiles, set)), TL::THREADS, smem, s>>>(p, g.guard, g.queue);
+    } else {
+        auto kern = fma_gemm_kernel<TL, T, AKC, BKC, PER_SM>;
+        BX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        kern<<<unsigned(tiles), TL::THREADS, smem, s>>>(p, g.guard);
+    }
     BX_CUDA(cudaGetLastError());
     count_launch();
     return BLASX_OK;
@@ -156,8 +165,10 @@ template <typename T> int launch_t(const Gemm &g, cudaStream_t s) {
 
 bool fma_preferred(const Gemm &g) {
     if (g.dt == DType::F32) return (g.N + 127) / 128 <= 65535;
-    // complex64: the 64x64 SIMT tile from four of them per SM on
-    return g.dt == DType::C64 && ((g.M + 63) / 64) * ((g.N + 63) / 64) < 4 * kSms && (g.N + 63) / 64 <= 65535;
+    // complex64: the 64x64 SIMT tile from three of them per two SMs on
+    // (1394 x 699 x 66, 242 tiles: 35 us, 45 with 32x32 tiles; 512^3, 64
+    // tiles: 113 against 35)
+    return g.dt == DType::C64 && 2 * ((g.M + 63) / 64) * ((g.N + 63) / 64) < 3 * kSms && (g.N + 63) / 64 <= 65535;
 }
 
 int launch_gemm_fma(const Gemm &g, cudaStream_t s) {
