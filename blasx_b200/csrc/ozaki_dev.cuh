@@ -3,7 +3,9 @@
 // slicing of FP64 / FP32 / complex operands into int8 residues, and the CRT
 // reconstruction with the alpha / beta epilogue. Each stage is a device body
 // over explicit block coordinates, shared by the standalone kernels
-// (ozaki.cu) and the serving executor (executor.cu). Everything here has
+// (ozaki.cu) and the serving executor (executor.cu) -- except the statistics
+// and the decision, which are stages of their own in the executor and one
+// launch in the standalone path (ozaki_stats.cuh). Everything here has
 // internal linkage: every translation unit that includes it holds its own
 // copy of the constant tables and uploads them itself (upload_tables).
 #pragma once
