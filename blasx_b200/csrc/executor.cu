@@ -15,6 +15,7 @@
 //   kScale    beta-scaling of a range of C (alpha == 0 or K == 0)
 //   kZero     clearing of an emulated request's statistics and error word
 //   kStats    row statistics of op(A) or op(B), a range of blocks
+//   kPair     the pair sample's partial sums, a range of chunks
 //   kDecide   the modulus count and norm bound (one CTA)
 //   kSlice    int8 residues of op(A) or op(B), a range of blocks
 //   kResidue  one 256 x 128 C tile for every modulus: the tcgen05 pipeline
@@ -77,6 +78,7 @@ enum Kind : int32_t {
     kNone = 0,
     kZero,
     kStats,
+    kPair,
     kDecide,
     kSlice,
     kResidue,
@@ -112,6 +114,7 @@ struct alignas(128) ReqDesc {
     // emulated
     oz::View va, vb;
     oz::RowStats sa, sb, sbd;
+    oz::PairSample pair;
     oz::Decision *dec;
     int *ea, *fb, *err;
     oz::SliceOut oy, ox;
@@ -282,6 +285,10 @@ __device__ __forceinline__ void emulated_task(const ReqDesc &d, const Task &t, i
             }
             break;
         }
+        case kPair:
+            for (int64_t c = t.first; c < t.first + t.count; ++c)
+                oz::pair_chunk_body<T>(d.pair, c, tid, reinterpret_cast<double *>(work));
+            break;
         case kSlice: {
             const oz::View &v = side ? d.vb : d.va;
             const oz::RowStats &st = side ? d.sb : d.sa;
@@ -401,9 +408,11 @@ __global__ void __launch_bounds__(kThreads, 1) executor_kernel(const ExecArgs a)
                 for (int64_t w = t.first + tid; w < t.first + t.count; w += kThreads) d.zero_ptr[w] = 0u;
                 break;
             case kDecide:
-                oz::decide_body(d.sa, d.M, d.sbd, d.N, d.K, d.unit, d.mode, d.forced, d.dec, tid, kThreads);
+                oz::decide_body(d.sa, d.M, d.sbd, d.N, d.K, d.unit, d.mode, d.forced, d.dec, d.pair, tid,
+                                kThreads);
                 break;
             case kStats:
+            case kPair:
             case kSlice:
             case kRecon:
                 if (dt == DType::F64) emulated_task<double>(d, t, tid, work);
@@ -839,6 +848,8 @@ int prepare(Executor *e, int slot, const Gemm &g, bool emulated, int mode, void 
         // the error word, the decision and the statistics, contiguous from the scratch's start
         d.zero_ptr = reinterpret_cast<uint32_t *>(pt.err);
         d.zero_words = int64_t((reinterpret_cast<char *>(pt.ea) - reinterpret_cast<char *>(pt.err)) / 4);
+        if (mode == 0 && d.forced == 0)  // (no chunks otherwise)
+            d.pair = oz::pair_sample(d.va, d.akc, d.vb, d.bkc, g.uplo, g.diag, 64, pt.pair);
         Stage zero, stats, decide, slice, residue, recon;
         add_tasks(zero, kZero, slot, 0, d.zero_words, spread(d.zero_words, 1 << 14, e->num_sms));
         for (int side = 0; side < (pl.alias ? 1 : 2); ++side) {
@@ -857,6 +868,7 @@ int prepare(Executor *e, int slot, const Gemm &g, bool emulated, int mode, void 
             const int64_t blocks = d.slice_gx[side] * (Rp / 64);
             add_tasks(slice, kSlice, slot, side, blocks, spread(blocks, 1, e->num_sms));
         }
+        add_tasks(stats, kPair, slot, 0, d.pair.chunks, 1);
         add_tasks(decide, kDecide, slot, 0, 1, 1);
         d.res_tiles_j = pl.Jx / oz::kTileJ;
         d.res_tiles_i = pl.Ip / oz::kTileI;

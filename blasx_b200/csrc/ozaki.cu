@@ -31,20 +31,35 @@ namespace {
 
 // ---- the standalone kernels: one body block per CUDA block -------------------
 
+// The pair sample's blocks come first: a row of the grid of an operand's own
+// launch (its chunks are at most the blocks along k).
 template <typename T, int ROLE>
 __global__ void __launch_bounds__(256, ROLE == 0 ? 4 : (ROLE == 1 ? 3 : 2)) slice_kc_kernel(View v, RowStats st, const Decision *dec, int *expo,
-                                                       SliceOut o) {
-    slice_kc_body<T, ROLE>(v, st, dec, expo, o, blockIdx.x, blockIdx.y, threadIdx.x);
+                                                       SliceOut o, const __grid_constant__ PairVeto pv) {
+    __shared__ double2 smem[kPairShared / 2];
+    const int row0 = pv.p.chunks ? 1 : 0;
+    if (blockIdx.y < row0) {
+        if (int(blockIdx.x) < pv.p.chunks) pair_veto_block<T>(pv, blockIdx.x, threadIdx.x, reinterpret_cast<double *>(smem));
+        return;
+    }
+    slice_kc_body<T, ROLE>(v, st, dec, expo, o, blockIdx.x, blockIdx.y - row0, threadIdx.x);
 }
 
 template <typename T, int ROLE>
 __global__ void __launch_bounds__(256, ROLE == 0 ? 4 : (ROLE == 1 ? 3 : 2)) slice_rc_kernel(View v, RowStats st, const Decision *dec, int *expo,
-                                                       SliceOut o) {
+                                                       SliceOut o, const __grid_constant__ PairVeto pv) {
     __shared__ __align__(16) unsigned char smem[slice_rc_smem_bytes<ROLE>()];
-    slice_rc_body<T, ROLE>(v, st, dec, expo, o, blockIdx.x, blockIdx.y, threadIdx.x, smem);
+    static_assert(sizeof smem >= kPairShared * sizeof(double), "the pair sample's stage");
+    const int row0 = pv.p.chunks ? 1 : 0;
+    if (blockIdx.y < row0) {
+        if (int(blockIdx.x) < pv.p.chunks) pair_veto_block<T>(pv, blockIdx.x, threadIdx.x, reinterpret_cast<double *>(smem));
+        return;
+    }
+    slice_rc_body<T, ROLE>(v, st, dec, expo, o, blockIdx.x, blockIdx.y - row0, threadIdx.x, smem);
 }
 
-// Both operands of a real GEMM: blocks [0, na) slice op(A), the others op(B).
+// Both operands of a real GEMM: after the pair sample's, blocks [0, na) slice
+// op(A), the others op(B).
 struct SliceSide {
     View v;
     RowStats st;
@@ -53,10 +68,13 @@ struct SliceSide {
     int gx;  // blocks along k
 };
 template <typename T, bool AKC, bool BKC>
-__global__ void __launch_bounds__(256, 4) slice_both_kernel(SliceSide a, SliceSide b, int na, const Decision *dec) {
-    __shared__ __align__(16) unsigned char smem[(AKC && BKC) ? 16 : slice_rc_smem_bytes<0>()];
-    const int i = blockIdx.x;
-    if (i < na) {
+__global__ void __launch_bounds__(256, 4) slice_both_kernel(SliceSide a, SliceSide b, int na, const Decision *dec,
+                                                            const __grid_constant__ PairVeto pv) {
+    __shared__ __align__(16) unsigned char smem[(AKC && BKC) ? kPairShared * sizeof(double) : slice_rc_smem_bytes<0>()];
+    const int i = int(blockIdx.x) - pv.p.chunks;
+    if (i < 0) {
+        pair_veto_block<T>(pv, blockIdx.x, threadIdx.x, reinterpret_cast<double *>(smem));
+    } else if (i < na) {
         if (AKC) slice_kc_body<T, 0>(a.v, a.st, dec, a.expo, a.o, i % a.gx, i / a.gx, threadIdx.x);
         else slice_rc_body<T, 0>(a.v, a.st, dec, a.expo, a.o, i % a.gx, i / a.gx, threadIdx.x, smem);
     } else {
@@ -146,14 +164,15 @@ int launch_stats(const oz::View &va, bool akc, const oz::RowStats &sa, const oz:
 
 template <typename T, int ROLE>
 int launch_slice(const oz::View &v, bool kc, const oz::RowStats &st, const oz::Decision *dec,
-                 int *expo, const oz::SliceOut &o, int64_t Kc, cudaStream_t s) {
+                 int *expo, const oz::SliceOut &o, int64_t Kc, const oz::PairVeto &pv, cudaStream_t s) {
+    const unsigned rows = unsigned(o.Rp / 64) + (pv.p.chunks ? 1 : 0);
     if (kc) {
-        dim3 grid(unsigned(Kc / 64), unsigned(o.Rp / 64));
-        oz::slice_kc_kernel<T, ROLE><<<grid, 256, 0, s>>>(v, st, dec, expo, o);
+        dim3 grid(unsigned(Kc / 64), rows);
+        oz::slice_kc_kernel<T, ROLE><<<grid, 256, 0, s>>>(v, st, dec, expo, o, pv);
     } else {
         const int kt = ROLE ? 32 : 64;
-        dim3 grid(unsigned(Kc / kt), unsigned(o.Rp / 64));
-        oz::slice_rc_kernel<T, ROLE><<<grid, 256, 0, s>>>(v, st, dec, expo, o);
+        dim3 grid(unsigned(Kc / kt), rows);
+        oz::slice_rc_kernel<T, ROLE><<<grid, 256, 0, s>>>(v, st, dec, expo, o, pv);
     }
     BX_CUDA(cudaGetLastError());
     count_launch();
@@ -165,21 +184,21 @@ int launch_slice(const oz::View &v, bool kc, const oz::RowStats &st, const oz::D
 // be too large.
 template <typename T>
 bool slice_both_fits(const oz::SliceOut &oa, const oz::SliceOut &ob, int64_t Kc) {
-    return (Kc / 64) * (oa.Rp / 64 + ob.Rp / 64) <= INT32_MAX;
+    return (Kc / 64) * (oa.Rp / 64 + ob.Rp / 64 + 1) <= INT32_MAX;
 }
 template <typename T>
 int launch_slice_both(const oz::View &va, bool akc, const oz::RowStats &sa, int *ea, const oz::SliceOut &oa,
                       const oz::View &vb, bool bkc, const oz::RowStats &sb, int *fb, const oz::SliceOut &ob,
-                      const oz::Decision *dec, int64_t Kc, cudaStream_t s) {
+                      const oz::Decision *dec, int64_t Kc, const oz::PairVeto &pv, cudaStream_t s) {
     const int gx = int(Kc / 64), na = int(gx * (oa.Rp / 64)), nb = int(gx * (ob.Rp / 64));
     const oz::SliceSide a{va, sa, ea, oa, gx}, b{vb, sb, fb, ob, gx};
-    const unsigned grid = unsigned(na) + unsigned(nb);
+    const unsigned grid = unsigned(pv.p.chunks) + unsigned(na) + unsigned(nb);
     if (akc) {
-        if (bkc) oz::slice_both_kernel<T, true, true><<<grid, 256, 0, s>>>(a, b, na, dec);
-        else oz::slice_both_kernel<T, true, false><<<grid, 256, 0, s>>>(a, b, na, dec);
+        if (bkc) oz::slice_both_kernel<T, true, true><<<grid, 256, 0, s>>>(a, b, na, dec, pv);
+        else oz::slice_both_kernel<T, true, false><<<grid, 256, 0, s>>>(a, b, na, dec, pv);
     } else {
-        if (bkc) oz::slice_both_kernel<T, false, true><<<grid, 256, 0, s>>>(a, b, na, dec);
-        else oz::slice_both_kernel<T, false, false><<<grid, 256, 0, s>>>(a, b, na, dec);
+        if (bkc) oz::slice_both_kernel<T, false, true><<<grid, 256, 0, s>>>(a, b, na, dec, pv);
+        else oz::slice_both_kernel<T, false, false><<<grid, 256, 0, s>>>(a, b, na, dec, pv);
     }
     BX_CUDA(cudaGetLastError());
     count_launch();
@@ -220,15 +239,23 @@ int ozaki_run(const Gemm &g, cudaStream_t s, int mode, void *ws, int num_sms, vo
 
     oz::SliceOut oy{Y, Ip, Kp, Kh, Ip * Kp};
     oz::SliceOut ox{X, Jp, Kp, Kh, Jx * Kp};
+    // auto mode: the pair sample, with the slices of the operand that has
+    // fewer rows (its row of blocks fits the grid). Its counters are the last
+    // words of op(A)'s flags, padded to a multiple of 64: the arrival counters
+    // of op(A)'s groups, one for eight rows, end before them.
+    oz::PairVeto none{}, pv{};
+    if (mode == 0 && oz::forced_moduli() == 0)
+        pv = oz::pair_veto(va, akc, vb, bkc, g.uplo, g.diag, pt, sb.flags - oz::kPairCounters, dec);
+    const bool pv_first = pl.alias || oy.Rp <= ox.Rp;
     if constexpr (CPLX) {
-        BX_TRY((launch_slice<T, 1>(va, akc, sa, dec, ea, oy, Kc, s)));
-        BX_TRY((launch_slice<T, 2>(vb, bkc, sb, dec, fb, ox, Kc, s)));
+        BX_TRY((launch_slice<T, 1>(va, akc, sa, dec, ea, oy, Kc, pv_first ? pv : none, s)));
+        BX_TRY((launch_slice<T, 2>(vb, bkc, sb, dec, fb, ox, Kc, pv_first ? none : pv, s)));
     } else {
         if (!pl.alias && slice_both_fits<T>(oy, ox, Kc)) {
-            BX_TRY(launch_slice_both<T>(va, akc, sa, ea, oy, vb, bkc, sb, fb, ox, dec, Kc, s));
+            BX_TRY(launch_slice_both<T>(va, akc, sa, ea, oy, vb, bkc, sb, fb, ox, dec, Kc, pv, s));
         } else {
-            BX_TRY((launch_slice<T, 0>(va, akc, sa, dec, ea, oy, Kc, s)));
-            if (!pl.alias) BX_TRY((launch_slice<T, 0>(vb, bkc, sb, dec, fb, ox, Kc, s)));
+            BX_TRY((launch_slice<T, 0>(va, akc, sa, dec, ea, oy, Kc, pv_first ? pv : none, s)));
+            if (!pl.alias) BX_TRY((launch_slice<T, 0>(vb, bkc, sb, dec, fb, ox, Kc, pv_first ? none : pv, s)));
         }
     }
     // residue GEMMs and reconstruction, in column panels of C when asked.

@@ -46,6 +46,8 @@ struct Decision {
     int q;         // norm exponent bound Q
     double estimate;  // estimated max normalised error (units of the dtype's u)
     int nonfinite;
+    int slices;       // nmod as the slices take it (nmod may yet become 0 beside them)
+    double spread;    // rho_A rho_B
     int pad;  // zero; arrival counter before the decision, tile counter of the fallback after it
 };
 

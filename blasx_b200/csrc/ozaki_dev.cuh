@@ -213,19 +213,169 @@ __device__ __forceinline__ void stats_rc_body(const View &v, const RowStats &st,
     if (bad) atomicOr(&st.flags[r], 1);
 }
 
+// ---- how the operands' large entries meet -----------------------------------
+//
+// Scaled integers carry an error of one size along a whole row, so an entry
+// of C is as accurate as its |A||B| is large against ||a_i||_2 ||b_j||_2. Each
+// operand's own statistics do not show that: columns of A in mixed units and
+// rows of B in the inverse units look even on both sides, and every product
+// pairs a large entry with a small one (half of them by 10^6: |A||B| is 10^-6
+// of the product of the norms, the emulated result 10^3 units off). So
+// kPairRows rows of op(A) and as many columns of op(B), spread over the
+// operands, are multiplied in magnitude, and the smallest
+//   n = sum_k |a_ik| |b_kj| / (||a_i||_2 ||b_j||_2)
+// over their pairs inside the output's triangle enters the estimate. Pairs
+// whose sum is zero have an exact zero in C and do not count.
+// What bounds it: latency (a few thousand scattered loads). So the k extent is
+// cut into chunks of kPairChunk, a block of 256 threads each with all loads of
+// a step in flight; the chunks' partial sums go to scratch and are added in
+// chunk order. The standalone path runs these blocks among those of the slices,
+// which hide them (PairVeto, ozaki_stats.cuh).
+constexpr int kPairRows = 32, kPairStep = 32, kPairChunk = 64;
+constexpr int kPairLd = kPairRows + 2;                            // row of a staged k
+constexpr int kPairShared = 2 * kPairStep * kPairLd;              // doubles
+constexpr int kPairPart = kPairRows * kPairRows + 2 * kPairRows;  // doubles per chunk: products, then sums of squares
+struct PairSample {
+    View v[2];       // op(A) rows, op(B) columns over k
+    int kc[2];       // k-contiguous source
+    int uplo;
+    int64_t diag;
+    int chunks;
+    int64_t kchunk;
+    double *part;    // [chunks][kPairPart]
+};
+
+inline PairSample pair_sample(const View &va, bool akc, const View &vb, bool bkc, int uplo, int64_t diag,
+                              int max_chunks, double *part) {
+    PairSample p;
+    p.v[0] = va;
+    p.v[1] = vb;
+    p.kc[0] = akc;
+    p.kc[1] = bkc;
+    p.uplo = uplo;
+    p.diag = diag;
+    const int64_t most = (va.K + kPairChunk - 1) / kPairChunk;
+    p.chunks = int(most < max_chunks ? most : max_chunks);
+    p.kchunk = (va.K + p.chunks - 1) / p.chunks;
+    p.part = part;
+    return p;
+}
+
+// Row s of an operand's sample: one in each of kPairRows equal stretches of
+// its R rows, at a place that changes from stretch to stretch.
+__device__ __forceinline__ int64_t pair_row(int s, int64_t R, int side) {
+    const int64_t lo = s * R / kPairRows, hi = (s + 1) * R / kPairRows;
+    return lo + ((hi - lo) * ((s * 20 + 7 + 11 * side) % kPairRows)) / kPairRows;
+}
+
+// One chunk, by 256 threads; sh: kPairShared doubles.
+template <typename T>
+__device__ __forceinline__ void pair_chunk_body(const PairSample &p, int64_t chunk, int tid, double *sh) {
+    const int64_t k0 = chunk * p.kchunk, k1 = min(p.v[0].K, k0 + p.kchunk);
+    const int lane = tid & 31, warp = tid >> 5;        // a warp loads rows warp, warp + 8, ... of both operands
+    const int i = 2 * (tid / 16), j = 2 * (tid % 16);  // this thread's 2 x 2 pairs
+    double ssq[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}}, sum[2][2] = {{0, 0}, {0, 0}};
+    for (int64_t k = k0; k < k1; k += kPairStep) {
+        __syncthreads();  // the last step has been read
+#pragma unroll
+        for (int sd = 0; sd < 2; ++sd)
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                double x = 0.0, y = 0.0;
+                if (k + lane < k1)
+                    load_elem<T>(p.v[sd], pair_row(warp + 8 * h, p.v[sd].R, sd), k + lane, p.kc[sd] != 0, x, y);
+                ssq[sd][h] = fma(x, x, fma(y, y, ssq[sd][h]));
+                sh[(sd * kPairStep + lane) * kPairLd + warp + 8 * h] = fabs(x) + fabs(y);
+            }
+        __syncthreads();
+#pragma unroll 8
+        for (int q = 0; q < kPairStep; ++q) {
+            const double2 a = *reinterpret_cast<const double2 *>(&sh[q * kPairLd + i]);
+            const double2 b = *reinterpret_cast<const double2 *>(&sh[(kPairStep + q) * kPairLd + j]);
+            sum[0][0] = fma(a.x, b.x, sum[0][0]);
+            sum[0][1] = fma(a.x, b.y, sum[0][1]);
+            sum[1][0] = fma(a.y, b.x, sum[1][0]);
+            sum[1][1] = fma(a.y, b.y, sum[1][1]);
+        }
+    }
+    double *w = p.part + chunk * kPairPart;
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int b = 0; b < 2; ++b) w[(i + a) * kPairRows + j + b] = sum[a][b];
+#pragma unroll
+    for (int sd = 0; sd < 2; ++sd)
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            double v = ssq[sd][h];
+            for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == 0) w[kPairRows * kPairRows + sd * kPairRows + warp + 8 * h] = v;
+        }
+}
+
+// The sum of n partial results: this thread's values e = tid, tid + 256, ...
+constexpr int kPairPer = (kPairPart + 255) / 256;
+__device__ __forceinline__ void pair_add(const double *in, int n, int tid, double (&v)[kPairPer]) {
+#pragma unroll
+    for (int q = 0; q < kPairPer; ++q) v[q] = 0;
+#pragma unroll 4
+    for (int c = 0; c < n; ++c, in += kPairPart)
+#pragma unroll
+        for (int q = 0; q < kPairPer; ++q) {
+            const int e = tid + 256 * q;
+            if (e < kPairPart) v[q] += __ldcg(in + e);
+        }
+}
+
+// The smallest n over the pairs from `count` partial results at `in` (256
+// threads; the result is in thread 0). 1e300 when no pair counts.
+__device__ __forceinline__ double pair_reduce(const PairSample &p, const double *in, int count, int tid, double *sh) {
+    static_assert(kPairRows * kPairRows % 256 == 0 && 2 * kPairRows <= 256, "a thread's last value is a sum of squares");
+    double v[kPairPer];
+    pair_add(in, count, tid, v);
+    __syncthreads();  // sh is free
+    if (tid < 2 * kPairRows) sh[tid] = sqrt(v[kPairPer - 1]);
+    __syncthreads();
+    double least = 1e300;
+#pragma unroll
+    for (int q = 0; q < kPairPer - 1; ++q) {
+        const int e = tid + 256 * q, i = e / kPairRows, j = e % kPairRows;
+        const int64_t d = pair_row(i, p.v[0].R, 0) - pair_row(j, p.v[1].R, 1);
+        if (p.uplo && (p.uplo == 1 ? d > p.diag : d < p.diag)) continue;
+        if (v[q] > 0) least = fmin(least, v[q] / (sh[i] * sh[kPairRows + j]));
+    }
+    for (int o = 16; o; o >>= 1) least = fmin(least, __shfl_xor_sync(0xffffffffu, least, o));
+    if (tid % 32 == 0) sh[2 * kPairRows + tid / 32] = least;
+    __syncthreads();
+    if (tid == 0)
+        for (int w = 1; w < 8; ++w) least = fmin(least, sh[2 * kPairRows + w]);
+    return least;
+}
+
+// The estimate E(N) of decide_body with the pairs in it. Rows that pair evenly
+// have n near 1 / (rho_A rho_B), which E(N) takes for granted, scattered by
+// chance; a smallest n below an eighth of that raises it in proportion.
+constexpr double kPairSlack = 8.0;
+__device__ __forceinline__ double paired_estimate(double est, double spread, double least) {
+    return est / fmin(1.0, kPairSlack * spread * least);
+}
+
 // Chooses the modulus count. Estimated max componentwise error, in units of
 // the output dtype's unit roundoff u:
 //   E(N) = C * rho_A * rho_B * 2^-q(N) / u,  rho = ||x||_2 sqrt(K) / ||x||_1,
 //   q(N) = min(Q_N, P + min_rows log2(||x||_2 / max|x|)),
 // calibrated on double-double references (C = 3). The smallest N with
 // E(N) <= 1/2 is taken; mode auto falls back to native (N = 0) when even
-// kMaxModuli does not reach it, mode ozaki takes kMaxModuli instead.
-// One block of nthreads (a multiple of 32, at most 1024) threads.
+// kMaxModuli does not reach it, or when the pair sample (ps; above) raises the
+// taken estimate over 1/2; mode ozaki takes kMaxModuli instead, whatever the
+// pairs are.
+// One block of nthreads = 256 threads.
 __device__ __forceinline__ void decide_body(const RowStats &sa, int64_t Ra, const RowStats &sb, int64_t Rb,
-                                           int64_t K, double unit, int mode, int forced, Decision *dec, int tid,
-                                           int nthreads) {
-    __shared__ double s_rho[2][32], s_h[2][32];
+                                           int64_t K, double unit, int mode, int forced, Decision *dec,
+                                           const PairSample &ps, int tid, int nthreads) {
+    __shared__ double s_rho[2][32], s_h[2][32], s_pair[2 * kPairRows + 8];
     __shared__ int s_bad[32];
+    const double least = ps.chunks ? pair_reduce(ps, ps.part, ps.chunks, tid, s_pair) : 1e300;
     double rho[2] = {0, 0}, h[2] = {1e300, 1e300};
     int bad = 0;
     for (int side = 0; side < 2; ++side) {
@@ -284,7 +434,12 @@ __device__ __forceinline__ void decide_body(const RowStats &sa, int64_t Ra, cons
     }
     if (!chosen && mode == 2) chosen = kMaxModuli;
     if (d.nonfinite) chosen = 0;  // Inf/NaN: the native kernel propagates them
-    d.nmod = chosen;
+    d.spread = ra * rb;
+    if (chosen && ps.chunks) {
+        est = paired_estimate(est, d.spread, least);
+        if (!(est <= 0.5)) chosen = 0;
+    }
+    d.nmod = d.slices = chosen;
     d.q = chosen ? c_crt.Q[chosen - kMinModuli] : 0;
     d.estimate = est;
     *dec = d;
@@ -510,7 +665,7 @@ __device__ __forceinline__ void slice_kc_comp(const View &v, int nmod, int e, in
 template <typename T, int ROLE>
 __device__ __forceinline__ void slice_kc_body(const View &v, const RowStats &st, const Decision *dec, int *expo,
                                               const SliceOut &o, int64_t bx, int64_t by, int tid) {
-    const int nmod = dec->nmod;
+    const int nmod = dec->slices;
     if (nmod == 0) return;
     const int Q = dec->q;
     const int64_t r = by * 64 + (tid >> 2);
@@ -546,7 +701,7 @@ __device__ __forceinline__ void slice_rc_body(const View &v, const RowStats &st,
     constexpr int COMP = KT * kRcLd;  // one component's tile
     int64_t *tile = static_cast<int64_t *>(smem);
     int *s_e = reinterpret_cast<int *>(tile + CPL * COMP);
-    const int nmod = dec->nmod;
+    const int nmod = dec->slices;
     if (nmod == 0) return;
     const int Q = dec->q;
     const int64_t r0 = by * 64, k0 = bx * KT;
@@ -1062,7 +1217,7 @@ Plan make_plan(const Gemm &g) {
     p.alias = aliased(g);
     p.Jp = p.alias ? p.Ip : pad(p.N, kTileJ);
     p.Jx = cplx ? 2 * p.Jp : p.Jp;  // X rows (Re block + Im block)
-    p.bytes = 256 * 16 + (3 * sizeof(double) + 2 * sizeof(int)) * size_t(p.M + p.N) +
+    p.bytes = 256 * 15 + (3 * sizeof(double) + 2 * sizeof(int)) * size_t(p.M + p.N) +
               sizeof(Decision) + sizeof(int) + size_t(L) * p.Ip * p.Kp +
               (p.alias ? 0 : size_t(L) * p.Jx * p.Kp) + size_t(L) * p.Jx * p.Ip;
     return p;
@@ -1079,6 +1234,8 @@ struct Parts {
     int *ea, *fb;
     int8_t *Y, *X;
     uint8_t *U;
+    double *pair;  // partial results of the pair sample
+    int64_t pair_slots;  // and how many there is room for
 };
 inline Parts carve_parts(const Gemm &g, const Plan &pl, void *ws) {
     const int64_t L = kMaxModuli;
@@ -1096,6 +1253,11 @@ inline Parts carve_parts(const Gemm &g, const Plan &pl, void *ws) {
     p.Y = cv.take<int8_t>(size_t(L) * pl.Ip * pl.Kp);
     p.X = pl.alias ? p.Y : cv.take<int8_t>(size_t(L) * pl.Jx * pl.Kp);
     p.U = cv.take<uint8_t>(size_t(L) * pl.Jx * pl.Ip);
+    // in U, which the residue GEMM is the first to write
+    p.pair = reinterpret_cast<double *>(p.U);
+    p.pair_slots = int64_t(L) * pl.Jx * pl.Ip / int64_t(kPairPart * sizeof(double));
+    static_assert(int64_t(kMaxModuli) * kTileJ * kTileI / int64_t(kPairPart * sizeof(double)) >= 64 + 8 + 1,
+                  "64 chunks, their groups and the result fit the smallest U");
     return p;
 }
 

@@ -6,16 +6,19 @@
 // of a few thousand rows too. An operand is cut into groups of rows (8 for a
 // k-contiguous source, one warp per row; 64 for a row-contiguous one, warps
 // striding over k) times chunks of k; the chunk count follows from the number
-// of groups, so that about kStatsBlocks blocks exist whatever the shape. Each
-// chunk leaves its partial sums in scratch, the block that arrives last at
-// its group adds them in chunk order (the result does not depend on timing),
-// and the block that arrives last of all reduces the groups and decides.
+// of groups, so that kStatsBlocks blocks exist where the least chunk allows it
+// (two k-contiguous operands of 2048 x 2048 make 1024). Each chunk leaves its
+// partial sums in scratch, the block that arrives last at its group adds them
+// in chunk order (the result does not depend on timing), and the block that
+// arrives last of all reduces the groups and decides.
 //
 // One thread per row over 512 k with atomics, a second launch for the other
 // operand and a one-block decision kernel took 81 + 12 + 16 us at 2048^3 and
 // 138 + 15 + 18 us for a complex128 product of 2401 x 1639 x 1203; see the
 // launch in ozaki.cu for what this form takes.
 #pragma once
+
+#include <algorithm>
 
 #include "ozaki_dev.cuh"
 
@@ -126,7 +129,8 @@ __device__ __forceinline__ void decide_warp(const StatsArgs &a, const double (&r
     if (!chosen && a.mode == 2) chosen = kMaxModuli;
     if (bad) chosen = 0;  // Inf/NaN: the native kernel propagates them
     Decision d;
-    d.nmod = chosen;
+    d.nmod = d.slices = chosen;
+    d.spread = ra * rb;
     d.q = chosen ? c_crt.Q[chosen - kMinModuli] : 0;
     d.estimate = est_at;
     d.nonfinite = bad;
@@ -334,6 +338,77 @@ template <typename T> __global__ void __launch_bounds__(kStatsThreads) stats_dec
         ratio[1] = ratio[0];
     }
     decide_warp(a, rho, ratio, ratio[0] < 0 || ratio[1] < 0, lane);
+}
+
+// ---- the pair sample beside the slices ------------------------------------------
+//
+// In auto mode the first blocks of a slice launch take the pair sample; the
+// last of them sets the modulus count to zero, so that the residue GEMM and
+// the reconstruction do nothing and the native kernel runs, when the operands'
+// large entries do not meet. (Decision::slices keeps the count for the slices
+// that run meanwhile.) As part of the statistics the sample's chain of loads
+// and hand-overs delayed the decision: 7.6 us at FP64 2048^3, 10.3 at FP32
+// 3001 x 1777 x 999. Beside the slices it costs less than 1 us there, and 6 us
+// where they are shorter than its chain (DSYRK 4000 x 1000: 22.6 -> 28.5). The chunks are added in two
+// levels, groups of 16 or the square root of their number.
+constexpr int kPairMaxGroup = 32, kPairCounters = kPairMaxGroup + 1;
+struct PairVeto {
+    PairSample p;  // no chunks: no sample
+    int group;     // chunks per group
+    int *arrive;   // zeroed: per group, then for the groups
+    Decision *dec;
+};
+// counters: kPairCounters words.
+inline PairVeto pair_veto(const View &va, bool akc, const View &vb, bool bkc, int uplo, int64_t diag,
+                          const Parts &pt, int *counters, Decision *dec) {
+    PairVeto a;
+    // (64 chunks fit the smallest scratch; slots for the groups and the result)
+    const int64_t room = std::max<int64_t>(64, pt.pair_slots - kPairCounters - 1);
+    a.p = pair_sample(va, akc, vb, bkc, uplo, diag, int(std::min<int64_t>(room, kPairMaxGroup * kPairMaxGroup)),
+                      pt.pair);
+    a.group = 16;
+    while (a.group * a.group < a.p.chunks) ++a.group;
+    a.arrive = counters;
+    a.dec = dec;
+    return a;
+}
+
+// Counts one arrival of `of` at `counter`; true in every thread of the block
+// that is the last one, which may then read what the others left.
+__device__ __forceinline__ bool last_arrival(int *counter, int of, int tid) {
+    __shared__ int s_last;
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) s_last = atomicAdd(counter, 1) == of - 1;
+    __syncthreads();
+    if (!s_last) return false;
+    __threadfence();
+    return true;
+}
+
+template <typename T>
+__device__ __noinline__ void pair_veto_block(const PairVeto &a, int chunk, int tid, double *sh) {
+    const PairSample &p = a.p;
+    if (a.dec->slices == 0) return;  // native already
+    const int per = a.group, groups = (p.chunks + per - 1) / per, group = chunk / per;
+    double *sums = p.part + int64_t(p.chunks) * kPairPart;
+    pair_chunk_body<T>(p, chunk, tid, sh);
+    const int n = min(per, p.chunks - group * per);
+    if (!last_arrival(a.arrive + group, n, tid)) return;
+    if (groups > 1) {
+        double v[kPairPer];
+        pair_add(p.part + int64_t(group) * per * kPairPart, n, tid, v);
+#pragma unroll
+        for (int q = 0; q < kPairPer; ++q)
+            if (tid + 256 * q < kPairPart) sums[int64_t(group) * kPairPart + tid + 256 * q] = v[q];
+        if (!last_arrival(a.arrive + kPairMaxGroup, groups, tid)) return;
+    }
+    const double least = groups > 1 ? pair_reduce(p, sums, groups, tid, sh) : pair_reduce(p, p.part, n, tid, sh);
+    if (tid == 0) {
+        const double est = paired_estimate(a.dec->estimate, a.dec->spread, least);
+        a.dec->estimate = est;
+        if (!(est <= 0.5)) a.dec->nmod = 0;
+    }
 }
 
 }  // namespace
