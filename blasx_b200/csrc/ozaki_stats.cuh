@@ -349,8 +349,9 @@ template <typename T> __global__ void __launch_bounds__(kStatsThreads) stats_dec
 // that run meanwhile.) As part of the statistics the sample's chain of loads
 // and hand-overs delayed the decision: 7.6 us at FP64 2048^3, 10.3 at FP32
 // 3001 x 1777 x 999. Beside the slices it costs less than 1 us there, and 6 us
-// where they are shorter than its chain (DSYRK 4000 x 1000: 22.6 -> 28.5). The chunks are added in two
-// levels, groups of 16 or the square root of their number.
+// where they are shorter than its chain (DSYRK 4000 x 1000: 22.6 -> 28.5). The
+// chunks are added in two levels, groups of 16 or the square root of their
+// number.
 constexpr int kPairMaxGroup = 32, kPairCounters = kPairMaxGroup + 1;
 struct PairVeto {
     PairSample p;  // no chunks: no sample

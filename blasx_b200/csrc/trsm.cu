@@ -155,7 +155,8 @@ __global__ void __launch_bounds__(kBlockThreads)
         const int m = FORWARD ? mm : kRows - 1 - mm;  // compile-time after unrolling
         if (32 * m >= bs) continue;
 #pragma unroll
-        for (int v = 0; v < NV; ++v) c[m][v] = Ar::add(Ar::mul(scale, rhs[v]), c[m][v]);
+        for (int v = 0; v < NV; ++v)  // (a row beyond bs stays zero whatever the scale: inf * 0 is not)
+            if (lane + 32 * m < bs) c[m][v] = Ar::add(Ar::mul(scale, rhs[v]), c[m][v]);
         if (FORWARD ? 32 * (m + 1) < bs : m > 0) load_rhs(FORWARD ? m + 1 : m - 1);
 #pragma unroll 1
         for (int h = 0; h < 2; ++h) {
