@@ -26,8 +26,13 @@ namespace {
 // ... of each.
 constexpr int kBlock = 256, kRows = kBlock / 32;
 constexpr int kBlockThreads = 256;
-constexpr int kPanel = 16;  // columns of S staged at a time
+constexpr int kSms = 148;
 constexpr int kPanelLd = kBlock + 1;
+// Columns of S staged at a time (PANEL): 16, and 8 for complex128 with more
+// CTAs than SMs, where two panels of 16 (135 KB) leave an SM one CTA (256 x
+// 4096 199 us, 163 with 8; 2048 x 8192 4.62 ms, 4.07). With an SM to itself a
+// CTA is better off with fewer barriers (2048 x 64: 498 us, 538 with 8).
+constexpr int kPanel = 16, kSmallPanel = 8;
 // Vectors per warp: 16 bytes of each row per lane (32 registers in all).
 template <typename T> struct Vecs {
     static constexpr int n = 16 / int(sizeof(T));
@@ -72,14 +77,14 @@ template <typename T> __device__ __forceinline__ void copy_or_zero(T *dst, const
 // launch instead of four substitutions of 64 rows with three updates between
 // them; every warp runs its own vectors, the rows after step k updated by all
 // lanes at once, and a step needs no barrier. S passes through shared memory
-// 16 columns at a time (cp.async, the next panel in flight), zero outside its
+// a few columns at a time (cp.async, the next panel in flight), zero outside its
 // triangle and beyond bs; the CTA's warps share it. Rows beyond bs are zero
 // vectors with a unit diagonal. FP64, 256 rows: 28.5 us for 2048 vectors (87
 // as four 64-row substitutions and their updates), 132 for 16384 (136); a
 // DTRSM of 4096 rows and 2048 vectors fell from 2083 to 1417 us. Four vectors
 // per lane and four warps per CTA took 79 us for 2048: with one warp per
 // scheduler every instruction's latency shows.
-template <typename T, bool FORWARD, bool UNIT>
+template <typename T, bool FORWARD, bool UNIT, int PANEL>
 __global__ void __launch_bounds__(kBlockThreads)
     trsm_block_kernel(const T *__restrict__ A, int64_t lda, T *__restrict__ C, int64_t ldc, int bs, int64_t nvec,
                       int left, int s_trans, int s_conj, T scale) {
@@ -88,41 +93,41 @@ __global__ void __launch_bounds__(kBlockThreads)
     static_assert(TH == kBlock, "a thread loads one row of a panel");
     extern __shared__ __align__(16) unsigned char smem[];
     T *P = reinterpret_cast<T *>(smem);            // P[buf][k][i]: S[i][k0 + k]
-    T *rdiag = P + 2 * kPanel * kPanelLd;          // 1 / S[k][k]
+    T *rdiag = P + 2 * PANEL * kPanelLd;          // 1 / S[k][k]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t v0 = (int64_t(blockIdx.x) * WARPS + warp) * NV;
 
     // panel at column k0 of S into buffer b. Untransposed: thread i copies
-    // row i, column after column (coalesced); transposed: 16 threads a row's
-    // 16 columns. Rows of 32-row groups that the panel's steps do not read
+    // row i, column after column (coalesced); transposed: adjacent threads a
+    // row's columns. Rows of 32-row groups that the panel's steps do not read
     // are skipped.
     auto load_panel = [&](int k0, int b) {
-        T *dst = P + b * kPanel * kPanelLd;
+        T *dst = P + b * PANEL * kPanelLd;
         const int g = k0 / 32 * 32;
         if (!s_trans) {
             const int i = tid;
             if (FORWARD ? i >= g : i < g + 32) {
                 const T *src = A + i + int64_t(k0) * lda;
 #pragma unroll
-                for (int k = 0; k < kPanel; ++k, src += lda) {
+                for (int k = 0; k < PANEL; ++k, src += lda) {
                     const bool in = i < bs && k0 + k < bs && (FORWARD ? i > k0 + k : i < k0 + k);
                     copy_or_zero(dst + k * kPanelLd + i, in ? src : A, in);
                 }
             }
         } else {
-            const int k = tid % kPanel, col = k0 + k;
-            const int i0 = (FORWARD ? g : 0) + tid / kPanel, i1 = FORWARD ? kBlock : g + 32;
+            const int k = tid % PANEL, col = k0 + k;
+            const int i0 = (FORWARD ? g : 0) + tid / PANEL, i1 = FORWARD ? kBlock : g + 32;
             const T *src = A + col + int64_t(i0) * lda;
 #pragma unroll 2
-            for (int i = i0; i < i1; i += TH / kPanel, src += int64_t(TH / kPanel) * lda) {
+            for (int i = i0; i < i1; i += TH / PANEL, src += int64_t(TH / PANEL) * lda) {
                 const bool in = i < bs && col < bs && (FORWARD ? i > col : i < col);
                 copy_or_zero(dst + k * kPanelLd + i, in ? src : A, in);
             }
         }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
-    const int first = FORWARD ? 0 : (bs - 1) / kPanel * kPanel;
-    load_panel(first, first / kPanel & 1);
+    const int first = FORWARD ? 0 : (bs - 1) / PANEL * PANEL;
+    load_panel(first, first / PANEL & 1);
     for (int i = tid; i < kBlock; i += TH) {
         T r = Ar::one();
         if (!UNIT && i < bs) {
@@ -159,18 +164,18 @@ __global__ void __launch_bounds__(kBlockThreads)
             if (lane + 32 * m < bs) c[m][v] = Ar::add(Ar::mul(scale, rhs[v]), c[m][v]);
         if (FORWARD ? 32 * (m + 1) < bs : m > 0) load_rhs(FORWARD ? m + 1 : m - 1);
 #pragma unroll 1
-        for (int h = 0; h < 2; ++h) {
-            const int half = FORWARD ? h : 1 - h, k0 = 32 * m + 16 * half;
+        for (int h = 0; h < 32 / PANEL; ++h) {
+            const int part = FORWARD ? h : 32 / PANEL - 1 - h, k0 = 32 * m + PANEL * part;
             if (k0 >= bs) continue;
             asm volatile("cp.async.wait_group 0;\n" ::: "memory");
             __syncthreads();  // the panel has landed, and every warp has left the other buffer
-            const int next = FORWARD ? k0 + kPanel : k0 - kPanel;
-            if (FORWARD ? next < bs : next >= 0) load_panel(next, next / kPanel & 1);
-            const T *panel = P + (k0 / kPanel & 1) * kPanel * kPanelLd + lane;
+            const int next = FORWARD ? k0 + PANEL : k0 - PANEL;
+            if (FORWARD ? next < bs : next >= 0) load_panel(next, next / PANEL & 1);
+            const T *panel = P + (k0 / PANEL & 1) * PANEL * kPanelLd + lane;
 #pragma unroll 4
-            for (int q = 0; q < kPanel; ++q) {
-                const int kq = FORWARD ? q : kPanel - 1 - q;
-                const int kk = 16 * half + kq;  // the lane owning row k
+            for (int q = 0; q < PANEL; ++q) {
+                const int kq = FORWARD ? q : PANEL - 1 - q;
+                const int kk = PANEL * part + kq;  // the lane owning row k
                 const T *col = panel + kq * kPanelLd;
                 T x[NV];
 #pragma unroll
@@ -213,14 +218,11 @@ __global__ void __launch_bounds__(kBlockThreads)
         }
 }
 
-template <typename T> constexpr size_t block_smem() {
-    return sizeof(T) * (2 * kPanel * kPanelLd + kBlock);
-}
-
-template <typename T, bool FORWARD, bool UNIT>
+template <typename T, bool FORWARD, bool UNIT, int PANEL = kPanel>
 int launch_block_k(const Trsm &t, int64_t lo, int64_t hi, cplx scale, int s_trans, cudaStream_t s) {
+    constexpr size_t smem = sizeof(T) * (2 * PANEL * kPanelLd + kBlock);
     static const cudaError_t attr = cudaFuncSetAttribute(
-        trsm_block_kernel<T, FORWARD, UNIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(block_smem<T>()));
+        trsm_block_kernel<T, FORWARD, UNIT, PANEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     BX_CUDA(attr);
     const int64_t nvec = t.left ? t.N : t.M;
     const T *A = static_cast<const T *>(t.A) + lo + lo * t.lda;
@@ -228,8 +230,11 @@ int launch_block_k(const Trsm &t, int64_t lo, int64_t hi, cplx scale, int s_tran
     constexpr int per = kBlockThreads / 32 * Vecs<T>::n;
     const int64_t blocks = (nvec + per - 1) / per;
     if (blocks > 0x7fffffff) return set_error(BLASX_ERR_UNSUPPORTED, "trsm: too many right-hand sides");
+    if constexpr (sizeof(T) == 16 && PANEL == kPanel) {
+        if (blocks > kSms) return launch_block_k<T, FORWARD, UNIT, kSmallPanel>(t, lo, hi, scale, s_trans, s);
+    }
     const bool conj = is_complex(t.dt) && t.trans == ConjT;
-    trsm_block_kernel<T, FORWARD, UNIT><<<unsigned(blocks), kBlockThreads, block_smem<T>(), s>>>(
+    trsm_block_kernel<T, FORWARD, UNIT, PANEL><<<unsigned(blocks), kBlockThreads, smem, s>>>(
         A, t.lda, C, t.ldb, int(hi - lo), nvec, t.left, s_trans, conj, from_cplx<T>(scale));
     BX_CUDA(cudaGetLastError());
     count_launch();
