@@ -155,6 +155,16 @@ constexpr TileModel kReal[] = {{1, 64, 64, 3, {0.55, 0.79, 0.87, 0}},
                                {0, 128, 128, 1, {0.78, 0, 0, 0}}};  // a single, nearly full wave
 constexpr TileModel kCplx[] = {{1, 64, 64, 2, {0.72, 0.86, 0, 0}}, {2, 32, 32, 4, {0.56, 0.76, 0.80, 0.83}}};
 
+// What a tile loses against its fraction on some layouts of the operands. Two
+// k-contiguous ones: 32x32 FP64 tiles 15%, 64x64 complex128 tiles 20% (3000 x
+// 3000 x 200: 634 us, 520 with 32x32 tiles; 2496 x 3072 x 83: 296 and 230;
+// the 64x128 tile, which served them before, 583 and 270).
+double layout_cost(const TileModel &m, double macs, const Gemm &g) {
+    const bool both_k = g.ta != NoTrans && g.tb == NoTrans;
+    if (macs != 1.0) return m.g == 1 && both_k ? 1.2 : 1.0;
+    return m.g == 2 && both_k ? 1.15 : 1.0;
+}
+
 template <int COUNT> Geometry pick_geometry(const TileModel (&models)[COUNT], double macs, const Gemm &g) {
     const int64_t sms = num_sms();
     Geometry best{models[0].g, 1};
@@ -166,9 +176,7 @@ template <int COUNT> Geometry pick_geometry(const TileModel (&models)[COUNT], do
         for (int s = 1; s == 1 || (s <= max_splits && g.K >= int64_t(32) * s && tiles < sms); s *= 2) {
             const int64_t ctas = tiles * s, round = sms * m.per_sm, rest = ctas % round;
             const int64_t n = (rest + sms - 1) / sms;
-            // one CTA, its pipe to itself; 32x32 tiles of two k-contiguous
-            // operands run 15% below the fraction of the other layouts
-            const double layout = m.g == 2 && macs == 1.0 && g.ta != NoTrans && g.tb == NoTrans ? 1.15 : 1.0;
+            const double layout = layout_cost(m, macs, g);
             const double share = layout * macs * m.bm * m.bn * double((g.K + s - 1) / s) / 64.0;
             const double t = share * (double(ctas / round) * m.per_sm / m.eff[m.per_sm - 1] +
                                       (n ? double(n) / m.eff[n - 1] : 0.0)) +

@@ -1,0 +1,89 @@
+"""GPU tests of the native kernels, one shape per tile and per k cut, with the
+launched kernel and its grid read back: the choice itself is tested, and the
+products of small integers are exact. k spans several turns of each tile's ring
+of stages."""
+import json
+import os
+import re
+import tempfile
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+T = {"d": torch.float64, "s": torch.float32, "z": torch.complex128, "c": torch.complex64}
+
+
+def launched(fn):
+    """(kernel name, blocks) of the native GEMM kernels that fn launches."""
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as p:
+        fn()
+        torch.cuda.synchronize()
+    with tempfile.TemporaryDirectory() as d:
+        p.export_chrome_trace(os.path.join(d, "trace.json"))
+        with open(os.path.join(d, "trace.json")) as f:
+            events = json.load(f)["traceEvents"]
+    return [(e["name"], e["args"]["grid"][0]) for e in events
+            if e.get("cat") == "kernel" and re.search(r"dmma_|fma_|sgemm128", e["name"])]
+
+
+def tile_of(name):
+    """The C tile of a native kernel, from its template arguments."""
+    m = re.search(r"dmma_\w+_kernel<(true|false), (?:true|false), (?:true|false), \d+, (\d)>", name)
+    if m:
+        g = int(m[2])
+        return {0: (64, 128) if m[1] == "true" else (128, 128), 1: (64, 64), 2: (32, 32), 3: (64, 48)}[g]
+    m = re.search(r"FmaTile<[^,]+, (\d+), (\d+), (\d+), ", name)
+    return (32 * int(m[1]), 32 * int(m[2])) + ((int(m[3]),) if "fma_gemm" in name else ())
+
+
+def integers(gen, rows, ld, dt, top):
+    x = torch.randint(-top, top + 1, (rows, ld), device="cuda", generator=gen, dtype=torch.int32)
+    if dt in "zc":
+        return torch.complex(x.to(torch.float64), torch.randint(-top, top + 1, (rows, ld), device="cuda", generator=gen,
+                                                                dtype=torch.int32).to(torch.float64)).to(T[dt])
+    return x.to(T[dt])
+
+
+@pytest.fixture
+def native(blx):
+    prev = blx.set_dgemm_mode(blx.MODE_NATIVE)
+    yield blx
+    blx.set_dgemm_mode(prev)
+
+
+def op(x, t):
+    return x.mT if t == "N" else (x.conj() if t == "C" else x)
+
+
+def run(blx, dt, ta, tb, m, n, k, pad, tile, cut):
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(m + n + k)
+    top = 2 if dt in "sc" else 8  # sums below 2^24 (2^53)
+    ra, ca = (m, k) if ta == "N" else (k, m)
+    rb, cb = (k, n) if tb == "N" else (n, k)
+    A, B, C = integers(gen, ca, ra + pad, dt, top), integers(gen, cb, rb + pad, dt, top), integers(gen, n, m + pad, dt, top)
+    out = C.clone()
+
+    def call():
+        rc = blx.gemm_device(ta, tb, m, n, k, 2.0, A, ra + pad, B, rb + pad, -1.0, out, m + pad, dtype=dt)
+        assert rc == blx.BLASX_OK, blx.last_error()
+
+    kernels = launched(call)
+    assert len(kernels) == 1, kernels
+    name, blocks = kernels[0]
+    assert tile_of(name) == tile, name
+    tiles = -(-m // tile[0]) * -(-n // tile[1])
+    assert blocks == tiles * cut and ("split" in name) == (cut > 1), (name, blocks, tiles)
+    wide = torch.complex128 if dt in "zc" else torch.float64
+    want = C.to(wide).clone()
+    want[:, :m] = (2 * (op(A[:, :ra].to(wide), ta) @ op(B[:, :rb].to(wide), tb)) - C[:, :m].to(wide).mT).mT
+    assert torch.equal(out.to(wide), want)
+
+
+@pytest.mark.parametrize("ta,tb,tile", [("N", "N", (64, 64)), ("C", "C", (64, 64)), ("N", "T", (64, 64)),
+                                        ("T", "N", (32, 32)), ("C", "N", (32, 32))])
+@pytest.mark.parametrize("shape", [(1408, 1664, 500), (1471, 1599, 83)])
+def test_complex128_tiles_by_layout(native, ta, tb, tile, shape):
+    run(native, "z", ta, tb, *shape, 0, tile, 1)
