@@ -75,11 +75,15 @@ int num_sms() {
     return sms;
 }
 
+// Shared memory of a CTA that leaves an SM two of them.
+constexpr size_t kTwoPerSm = 100 * 1024;
+
 template <bool CPLX, bool AKC, bool BKC, int KI, int G>
-int launch_cfg(const DmmaParams &p, int splits, cudaStream_t s) {
+int launch_cfg(const DmmaParams &p, int splits, cudaStream_t s, size_t least_smem) {
     using TL = Tile<CPLX, G>;
-    constexpr size_t smem = dmma_smem_bytes<CPLX, AKC, BKC, G>();
-    static_assert(smem <= 227 * 1024, "shared memory budget");
+    constexpr size_t need = dmma_smem_bytes<CPLX, AKC, BKC, G>();
+    static_assert(need <= 227 * 1024, "shared memory budget");
+    const size_t smem = std::max(need, least_smem);
     const int64_t tiles = int64_t(p.tiles_m) * p.tiles_n;
     if constexpr (G == 2) {
         if (splits > 1) {
@@ -105,7 +109,7 @@ int launch_cfg(const DmmaParams &p, int splits, cudaStream_t s) {
     auto kern = dmma_gemm_kernel<CPLX, AKC, BKC, KI, G>;
     int64_t grid = tiles;
     if constexpr (G != 0 && (CPLX || KI == 16)) {
-        const int64_t set = int64_t(TL::PER_SM) * num_sms();
+        const int64_t set = int64_t(least_smem ? 2 : TL::PER_SM) * num_sms();
         if (p.guard && p.queue && tiles <= 4 * set) {
             kern = dmma_queue_kernel<CPLX, AKC, BKC, KI, G>;
             grid = std::min(tiles, set);
@@ -131,7 +135,7 @@ int dmma_k() {
 
 // The tile geometry and the k split of one problem.
 struct Geometry {
-    int g, splits;
+    int g, splits, per_sm;
 };
 
 // Chosen by the estimated time in SM cycles. An SM does 64 FP64 multiply-adds
@@ -149,25 +153,46 @@ struct TileModel {
     double eff[4];
 };
 constexpr double kSplitCycles = 8000.0;
+// (64x64 FP64 tiles also two to an SM, by more shared memory than they need:
+// 585 of them are two such rounds, but one of three per SM and a third of one
+// that reaches 55%.)
 constexpr TileModel kReal[] = {{1, 64, 64, 3, {0.55, 0.79, 0.87, 0}},
+                               {1, 64, 64, 2, {0.55, 0.79, 0, 0}},
                                {3, 64, 48, 4, {0.53, 0.73, 0.77, 0.85}},
                                {2, 32, 32, 4, {0.43, 0.61, 0.70, 0.72}},
                                {0, 128, 128, 1, {0.78, 0, 0, 0}}};  // a single, nearly full wave
 constexpr TileModel kCplx[] = {{1, 64, 64, 2, {0.72, 0.86, 0, 0}}, {2, 32, 32, 4, {0.56, 0.76, 0.80, 0.83}}};
 
-// What a tile loses against its fraction on some layouts of the operands. Two
-// k-contiguous ones: 32x32 FP64 tiles 15%, 64x64 complex128 tiles 20% (3000 x
-// 3000 x 200: 634 us, 520 with 32x32 tiles; 2496 x 3072 x 83: 296 and 230;
-// the 64x128 tile, which served them before, 583 and 270).
-double layout_cost(const TileModel &m, double macs, const Gemm &g) {
-    const bool both_k = g.ta != NoTrans && g.tb == NoTrans;
-    if (macs != 1.0) return m.g == 1 && both_k ? 1.2 : 1.0;
-    return m.g == 2 && both_k ? 1.15 : 1.0;
+// Whether an operand with this base and leading dimension is copied 16 bytes
+// at a time (as DmmaParams::vec_a).
+bool wide_copies(const void *p, int64_t ld) { return ld % 2 == 0 && reinterpret_cast<uintptr_t>(p) % 16 == 0; }
+
+// What a tile loses against its fraction on some layouts of the operands, with
+// n CTAs of it per SM.
+// Two k-contiguous operands: 32x32 FP64 tiles 15%, 64x64 complex128 tiles 20%
+// (3000 x 3000 x 200: 634 us, 520 with 32x32 tiles; 2496 x 3072 x 83: 296 and
+// 230; the 64x128 tile, which served them before, 583 and 270).
+// FP64 operands that are m- or n-contiguous and copied 8 bytes at a time (odd
+// leading dimension): a smaller tile copies more of them per multiply-add, 6%
+// each against 64x64 (1000^3 NT: 32x32 tiles 111 us, 64x64 95; with even ones
+// 89 and 85).
+// 64x48 tiles of two such operands (NT) cover their latencies badly with one
+// or two CTAs per SM, whatever the copies (1003 x 777 x 641, odd: 70.5 us,
+// 64x64 64.2).
+double layout_cost(const TileModel &m, double macs, const Gemm &g, int64_t n) {
+    const bool a_k = g.ta != NoTrans, b_k = g.tb == NoTrans;
+    if (macs != 1.0) return m.g == 1 && a_k && b_k ? 1.2 : 1.0;
+    if (m.g != 2 && m.g != 3) return 1.0;
+    const int narrow = (!a_k && !wide_copies(g.A, g.lda)) + (!b_k && !wide_copies(g.B, g.ldb));
+    double cost = 1.0 + (m.g == 2 ? 0.06 : 0.065) * narrow;
+    if (m.g == 2 && a_k && b_k) cost *= 1.15;
+    if (m.g == 3 && !a_k && !b_k && n <= 2) cost *= 1.12;
+    return cost;
 }
 
 template <int COUNT> Geometry pick_geometry(const TileModel (&models)[COUNT], double macs, const Gemm &g) {
     const int64_t sms = num_sms();
-    Geometry best{models[0].g, 1};
+    Geometry best{models[0].g, 1, models[0].per_sm};
     double best_t = 1e300;
     for (const TileModel &m : models) {
         int64_t tiles = ((g.M + m.bm - 1) / m.bm) * ((g.N + m.bn - 1) / m.bn);
@@ -176,14 +201,14 @@ template <int COUNT> Geometry pick_geometry(const TileModel (&models)[COUNT], do
         for (int s = 1; s == 1 || (s <= max_splits && g.K >= int64_t(32) * s && tiles < sms); s *= 2) {
             const int64_t ctas = tiles * s, round = sms * m.per_sm, rest = ctas % round;
             const int64_t n = (rest + sms - 1) / sms;
-            const double layout = layout_cost(m, macs, g);
-            const double share = layout * macs * m.bm * m.bn * double((g.K + s - 1) / s) / 64.0;
-            const double t = share * (double(ctas / round) * m.per_sm / m.eff[m.per_sm - 1] +
-                                      (n ? double(n) / m.eff[n - 1] : 0.0)) +
+            const double share = macs * m.bm * m.bn * double((g.K + s - 1) / s) / 64.0;
+            const double t = share * (layout_cost(m, macs, g, m.per_sm) * double(ctas / round) * m.per_sm /
+                                          m.eff[m.per_sm - 1] +
+                                      (n ? layout_cost(m, macs, g, n) * double(n) / m.eff[n - 1] : 0.0)) +
                              (s > 1 ? kSplitCycles : 0.0);
             if (t < best_t) {
                 best_t = t;
-                best = Geometry{m.g, s};
+                best = Geometry{m.g, s, m.per_sm};
             }
         }
     }
@@ -204,15 +229,17 @@ int forced_tile() {
     return forced;
 }
 
-template <bool CPLX, int KI, int G> int launch_g(const Gemm &g, int splits, cudaStream_t s) {
+template <bool CPLX, int KI, int G> int launch_g(const Gemm &g, int splits, cudaStream_t s, size_t least_smem = 0) {
     const DmmaParams p = make_params<CPLX, G>(g);
     if (int64_t(p.tiles_m) * p.tiles_n * splits > INT32_MAX)
         return set_error(BLASX_ERR_UNSUPPORTED, "DMMA grid too large");
     const bool akc = g.ta != NoTrans;  // op(A) = A^T: stored K x M, k contiguous
     const bool bkc = g.tb == NoTrans;  // op(B) = B: stored K x N, k contiguous
     if (akc)
-        return bkc ? launch_cfg<CPLX, true, true, KI, G>(p, splits, s) : launch_cfg<CPLX, true, false, KI, G>(p, splits, s);
-    return bkc ? launch_cfg<CPLX, false, true, KI, G>(p, splits, s) : launch_cfg<CPLX, false, false, KI, G>(p, splits, s);
+        return bkc ? launch_cfg<CPLX, true, true, KI, G>(p, splits, s, least_smem)
+                   : launch_cfg<CPLX, true, false, KI, G>(p, splits, s, least_smem);
+    return bkc ? launch_cfg<CPLX, false, true, KI, G>(p, splits, s, least_smem)
+               : launch_cfg<CPLX, false, false, KI, G>(p, splits, s, least_smem);
 }
 
 template <int G> int launch_k(const Gemm &g, cudaStream_t s) {
@@ -225,10 +252,10 @@ template <int G> int launch_k(const Gemm &g, cudaStream_t s) {
 
 int launch_real(const Gemm &g, cudaStream_t s) {
     Geometry x = pick_geometry(kReal, 1.0, g);
-    if (forced_tile() >= 0) x = Geometry{forced_tile(), 1};
+    if (forced_tile() >= 0) x = Geometry{forced_tile(), 1, 0};
     switch (x.g) {
         case 0: return launch_k<0>(g, s);
-        case 1: return launch_k<1>(g, s);
+        case 1: return x.per_sm == 2 ? launch_g<false, 16, 1>(g, 1, s, kTwoPerSm) : launch_k<1>(g, s);
         case 3: return launch_g<false, 16, 3>(g, 1, s);
         default: return launch_g<false, 16, 2>(g, x.splits, s);
     }

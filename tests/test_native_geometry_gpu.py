@@ -87,3 +87,13 @@ def run(blx, dt, ta, tb, m, n, k, pad, tile, cut):
 @pytest.mark.parametrize("shape", [(1408, 1664, 500), (1471, 1599, 83)])
 def test_complex128_tiles_by_layout(native, ta, tb, tile, shape):
     run(native, "z", ta, tb, *shape, 0, tile, 1)
+
+
+@pytest.mark.parametrize("ta,tb,shape,pad,tile", [
+    ("N", "T", (1000, 1000, 1000), 0, (32, 32)), ("N", "T", (1000, 1000, 1000), 1, (64, 64)),  # 8-byte copies
+    ("T", "T", (1000, 1000, 1000), 1, (64, 64)), ("N", "N", (1000, 1000, 1000), 1, (64, 64)),
+    ("N", "T", (1003, 777, 641), 0, (32, 32)),
+    ("N", "N", (1003, 777, 641), 0, (64, 48)),
+])
+def test_fp64_tiles_by_copy_width(native, ta, tb, shape, pad, tile):
+    run(native, "d", ta, tb, *shape, pad, tile, 1)
