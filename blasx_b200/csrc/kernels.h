@@ -36,6 +36,9 @@ int device_gemm(const Gemm &g, cudaStream_t s);
 // takes it where fma_preferred).
 bool fma_preferred(const Gemm &g);
 int launch_gemm_fma(const Gemm &g, cudaStream_t s);
+// FP32 with 128 x 128 tiles (launch_gemm_simt takes it where sgemm128_preferred).
+bool sgemm128_preferred(const Gemm &g);
+int launch_sgemm128(const Gemm &g, cudaStream_t s);
 // Triangular solve on device operands (t.A, t.B device pointers): recursive
 // halving into device_gemm updates (native or emulated by the precision
 // mode) and a substitution kernel for blocks of <= 256 rows. Sets *emulated

@@ -142,6 +142,7 @@ template <typename T> int launch_scale_t(const Gemm &g, cudaStream_t s) {
 }  // namespace
 
 int launch_gemm_simt(const Gemm &g, cudaStream_t s) {
+    if (sgemm128_preferred(g)) return launch_sgemm128(g, s);
     if (fma_preferred(g) && g.M <= INT32_MAX && g.N <= INT32_MAX && g.K <= INT32_MAX) return launch_gemm_fma(g, s);
     switch (g.dt) {
         case DType::F32: return launch_simt_t<float>(g, s);

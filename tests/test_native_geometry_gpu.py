@@ -34,8 +34,10 @@ def tile_of(name):
     if m:
         g = int(m[2])
         return {0: (64, 128) if m[1] == "true" else (128, 128), 1: (64, 64), 2: (32, 32), 3: (64, 48)}[g]
+    if "sgemm128" in name:
+        return 128, 128
     m = re.search(r"FmaTile<[^,]+, (\d+), (\d+), (\d+), ", name)
-    return (32 * int(m[1]), 32 * int(m[2])) + ((int(m[3]),) if "fma_gemm" in name else ())
+    return 32 * int(m[1]), 32 * int(m[2])
 
 
 def integers(gen, rows, ld, dt, top):
@@ -74,7 +76,7 @@ def run(blx, dt, ta, tb, m, n, k, pad, tile, cut):
     assert len(kernels) == 1, kernels
     name, blocks = kernels[0]
     assert tile_of(name) == tile, name
-    tiles = -(-m // tile[0]) * -(-n // tile[1])
+    tiles = -(-m // tile[0]) * (1 if "sgemm128" in name else -(-n // tile[1]))  # (the grid's first extent)
     assert blocks == tiles * cut and ("split" in name) == (cut > 1), (name, blocks, tiles)
     wide = torch.complex128 if dt in "zc" else torch.float64
     want = C.to(wide).clone()
@@ -97,3 +99,36 @@ def test_complex128_tiles_by_layout(native, ta, tb, tile, shape):
 ])
 def test_fp64_tiles_by_copy_width(native, ta, tb, shape, pad, tile):
     run(native, "d", ta, tb, *shape, pad, tile, 1)
+
+
+@pytest.mark.parametrize("ta,tb", [("N", "N"), ("N", "T"), ("T", "N"), ("T", "T")])
+@pytest.mark.parametrize("shape,pad,tile", [((2500, 2492, 300), 1, (128, 128)), ((2500, 2492, 300), 0, (64, 64)),
+                                            ((2170, 2165, 257), 0, (128, 128)), ((2500, 2492, 250), 1, (64, 64)),
+                                            ((2400, 2400, 300), 1, (64, 64))])
+def test_fp32_tiles_by_copy_width(native, ta, tb, shape, pad, tile):
+    m, n, k = shape
+    run(native, "s", ta, tb, m, n, k, pad, tile, 1)
+
+
+def test_fp32_large_tile_as_the_fallback(blx):
+    # operands of wide spread with odd leading dimensions: the decision on the
+    # device leaves the call to the native kernel, bit for bit
+    m, n, k = 2170, 2165, 300
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(4)
+
+    def wide(cols, ld):
+        x = torch.rand((cols, ld), device="cuda", generator=gen) - 0.5
+        return x * torch.exp(6 * torch.randn((cols, ld), device="cuda", generator=gen))
+
+    A, B, C = wide(k, m + 1), wide(n, k + 1), wide(n, m + 1)
+    outs = []
+    for mode, path in ((blx.MODE_AUTO, 4), (blx.MODE_NATIVE, 1)):
+        prev = blx.set_dgemm_mode(mode)
+        out = C.clone()
+        kernels = launched(lambda: blx.gemm_device("N", "N", m, n, k, 1.5, A, m + 1, B, k + 1, -0.5, out, m + 1, dtype="s"))
+        blx.set_dgemm_mode(prev)
+        assert blx.call_stats()["path"] == path
+        assert tile_of(kernels[-1][0]) == (128, 128)
+        outs.append(out)
+    assert torch.equal(*outs)
