@@ -157,7 +157,7 @@ constexpr double kSplitCycles = 8000.0;
 // 585 of them are two such rounds, but one of three per SM and a third of one
 // that reaches 55%.)
 constexpr TileModel kReal[] = {{1, 64, 64, 3, {0.55, 0.79, 0.87, 0}},
-                               {1, 64, 64, 2, {0.55, 0.79, 0, 0}},
+                               {1, 64, 64, 2, {0.55, 0.77, 0, 0}},
                                {3, 64, 48, 4, {0.53, 0.73, 0.77, 0.85}},
                                {2, 32, 32, 4, {0.43, 0.61, 0.70, 0.72}},
                                {0, 128, 128, 1, {0.78, 0, 0, 0}}};  // a single, nearly full wave

@@ -132,3 +132,51 @@ def test_fp32_large_tile_as_the_fallback(blx):
         assert tile_of(kernels[-1][0]) == (128, 128)
         outs.append(out)
     assert torch.equal(*outs)
+
+
+@pytest.mark.parametrize("dt,ta,tb,shape,pad,tile,cut", [
+    ("d", "N", "N", (1408, 1664, 500), 0, (128, 128), 1), ("d", "T", "N", (1408, 1664, 500), 0, (128, 128), 1),
+    ("d", "N", "T", (1408, 1664, 500), 1, (128, 128), 1),
+    ("d", "N", "N", (1300, 1301, 1302), 0, (64, 64), 1), ("d", "T", "T", (1300, 1301, 1302), 1, (64, 64), 1),
+    ("d", "T", "T", (951, 2478, 338), 1, (64, 64), 1),  # two CTAs per SM
+    ("d", "T", "N", (1003, 777, 641), 0, (64, 48), 1), ("d", "N", "T", (300, 257, 60), 0, (32, 32), 1),
+    ("d", "T", "N", (35, 59, 253), 0, (32, 32), 4), ("d", "N", "N", (300, 299, 500), 1, (32, 32), 4),
+    ("d", "N", "T", (30, 32, 261), 0, (32, 32), 8), ("d", "T", "T", (100, 130, 300), 1, (32, 32), 8),
+    ("d", "N", "N", (96, 64, 1990), 0, (32, 32), 16), ("d", "T", "N", (33, 31, 700), 1, (32, 32), 16),
+    ("z", "T", "T", (41, 30, 133), 0, (32, 32), 4), ("z", "N", "N", (100, 130, 300), 0, (32, 32), 8),
+    ("z", "C", "N", (100, 130, 300), 1, (32, 32), 8), ("z", "N", "T", (160, 160, 700), 0, (32, 32), 16),
+    ("z", "C", "C", (200, 190, 700), 1, (32, 32), 16), ("z", "N", "N", (300, 300, 100), 0, (32, 32), 1),
+    ("s", "N", "N", (320, 257, 190), 0, (32, 32), 1), ("s", "T", "T", (700, 640, 128), 1, (32, 32), 1),
+    ("s", "T", "N", (1400, 1300, 333), 0, (64, 64), 1), ("s", "N", "T", (1400, 1300, 333), 1, (64, 64), 1),
+    ("s", "N", "N", (64, 96, 600), 0, (32, 32), 2), ("s", "T", "N", (61, 95, 1100), 1, (32, 32), 4),
+    ("s", "N", "T", (64, 96, 2100), 0, (32, 32), 8), ("s", "T", "T", (61, 95, 4200), 0, (32, 32), 16),
+    ("c", "N", "N", (500, 500, 60), 0, (32, 32), 1), ("c", "C", "T", (600, 620, 100), 1, (32, 32), 1),
+    ("c", "N", "C", (64, 96, 130), 0, (32, 32), 2), ("c", "T", "N", (211, 300, 257), 1, (32, 32), 4),
+    ("c", "C", "N", (61, 95, 520), 0, (32, 32), 8), ("c", "N", "T", (64, 96, 1030), 0, (32, 32), 16),
+])
+def test_every_tile_and_cut(native, dt, ta, tb, shape, pad, tile, cut):
+    run(native, dt, ta, tb, *shape, pad, tile, cut)
+
+
+@pytest.mark.parametrize("uplo", ["U", "L"])
+@pytest.mark.parametrize("n,k,trans,tile", [(1901, 300, "N", (128, 128)), (1355, 300, "N", (64, 64)), (1537, 300, "N", (64, 48)),
+                                            (1089, 300, "T", (64, 48)), (1348, 91, "T", (64, 64)), (2118, 90, "T", (128, 128)),
+                                            (300, 300, "N", (32, 32)), (200, 700, "T", (32, 32))])
+def test_triangular_output(native, uplo, n, k, trans, tile):
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(n)
+    rows, cols = (n, k) if trans == "N" else (k, n)
+    A, C = integers(gen, cols, rows, "d", 8), integers(gen, n, n, "d", 8)
+    out = C.clone()
+
+    def call():
+        rc = native.dsyrk_device(uplo, trans, n, k, 2.0, A, rows, -1.0, out, n)
+        assert rc == native.BLASX_OK, native.last_error()
+
+    kernels = launched(call)
+    assert len(kernels) == 1 and tile_of(kernels[0][0]) == tile, kernels
+    X = op(A, trans)
+    full = 2 * (X @ X.mT) - C.mT
+    keep = torch.ones_like(full, dtype=torch.bool)
+    keep = keep.tril() if uplo == "L" else keep.triu()
+    assert torch.equal(out, torch.where(keep, full, C.mT).mT)
