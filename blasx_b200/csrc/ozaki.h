@@ -8,7 +8,7 @@
 //      rounded to an integer (|a'| < 2^62, row 2-norm < 2^Q) so that every
 //      dot product of scaled rows is bounded by M/4, M = prod of the moduli;
 //   2. for each modulus m_l (pairwise coprime, <= 256) the scaled integers are
-//      reduced to symmetric residues in int8;
+//      reduced to int8 residues;
 //   3. one INT8 GEMM per modulus on the tcgen05 tensor cores accumulates in
 //      INT32 exactly (|residue| <= 128, K <= 65536); its epilogue reduces the
 //      accumulator mod m_l to a uint8 residue;

@@ -581,7 +581,7 @@ struct SliceOut {
     int64_t plane;   // bytes per modulus plane
 };
 
-// Packs the symmetric residues of 16 consecutive elements for modulus L.
+// Packs the residues of 16 consecutive elements for modulus L.
 template <int L> __device__ __forceinline__ uint4 pack16(const Digits (&x)[16]) {
     uint32_t w[4];
 #pragma unroll

@@ -9,7 +9,7 @@ of floating-point matrix multiplication using an integer modular technique"
 1. each row of A / column of B is scaled by a power of two and rounded to an
    integer, |a'| < 2^P and ||a'_i||_2 < 2^Q, so every scaled dot product is
    below M / 4 (M = product of the moduli);
-2. symmetric residues of the scaled integers for each modulus;
+2. int8 residues of the scaled integers for each modulus;
 3. one integer GEMM per modulus, reduced mod m;
 4. the Chinese remainder theorem recovers the exact scaled product, which is
    unscaled to floating point.
@@ -20,6 +20,7 @@ operands: the check ``emulate(..., verify=True)`` asserts it.
 from __future__ import annotations
 
 import math
+from fractions import Fraction
 
 import numpy as np
 
@@ -170,13 +171,18 @@ def crt_fp64(u, tables) -> float:
 
 
 # ---- the device's residue computation, restated --------------------------------
-# The slicing kernels (blasx_b200/csrc/ozaki_dev.cuh: residue_s) take the
-# symmetric residue of a scaled integer v (|v| < 2^62) for an odd modulus m
-# from the eight bytes b_k of the biased value v + 2^62: two byte dot products
-# against the constants 2^(8k) mod m plus -2^62 mod m give s = v (mod m); with
+# The slicing kernels (blasx_b200/csrc/ozaki_dev.cuh: residue_s) take a residue
+# of a scaled integer v (|v| < 2^62) from the eight bytes b_k of the biased
+# value v + 2^62: two byte dot products against the constants 2^(8k) mod m plus
+# -2^62 mod m give s = v (mod m).
+# ``residue_bytes`` is the symmetric residue by an integer quotient: with
 # h = (m - 1) / 2 and t = s + h < 2^20, the quotient q of t by m is the high
-# word of s * ceil(2^32 / m) + h * ceil(2^32 / m), and s - q m lies in [-h, h].
-# For m = 256 the residue is the low byte of v.
+# word of s * ceil(2^32 / m) + h * ceil(2^32 / m), and s - q m lies in [-h, h];
+# for m = 256 it is the low byte of v. The device does that for m = 256 and 255.
+# ``residue_fp32`` is its form for every smaller modulus: the quotient by FP32
+# multiply-adds on F = base + s, base a multiple of 256 m. The quotient may be
+# one off the nearest, so the residue lies in [-h - 1, h + 1].
+# ``device_residue`` is the one that the device computes.
 
 def residue_bytes(v: int, m: int) -> int:
     a = v + (1 << 62)
@@ -191,3 +197,22 @@ def residue_bytes(v: int, m: int) -> int:
     q = (s * magic + h * magic) >> 32
     assert q == (s + h) // m
     return s - q * m
+
+
+def residue_fp32(v: int, m: int) -> int:
+    a = v + (1 << 62)
+    s = sum(((a >> (8 * k)) & 255) * ((1 << (8 * k)) % m) for k in range(8)) + (m - (1 << 62) % m) % m
+    base = 256 * m * -(-12582912 // (256 * m))
+    F = base + s
+    assert 1 << 23 <= F < 1 << 24  # an exact float whose unit is one
+    # one FMA onto 1.5 * 2^23 rounds to an integer, half to even
+    t = round(Fraction(float(np.float32(1.0) / np.float32(m))) * F + 12582912)
+    q = t - (12582912 + base // m)
+    out = F - q * m
+    assert 1 << 23 <= t < 1 << 24 and abs(q) < 1 << 24 and 1 << 23 <= out < 1 << 24
+    r = out & 255
+    return r - 256 if r >= 128 else r
+
+
+def device_residue(v: int, m: int) -> int:
+    return residue_bytes(v, m) if m >= 255 else residue_fp32(v, m)
