@@ -145,7 +145,7 @@ int launch_gemm_simt(const Gemm &g, cudaStream_t s) {
     if (sgemm128_preferred(g)) return launch_sgemm128(g, s);
     if (fma_preferred(g) && g.M <= INT32_MAX && g.N <= INT32_MAX && g.K <= INT32_MAX) return launch_gemm_fma(g, s);
     switch (g.dt) {
-        case DType::F32: return launch_simt_t<float>(g, s);
+        case DType::F32: return set_error(BLASX_ERR_UNSUPPORTED, "N too large for SIMT grid");
         case DType::F64: return launch_simt_t<double>(g, s);
         case DType::C64: return launch_simt_t<c2>(g, s);
         default: return launch_simt_t<z2>(g, s);
