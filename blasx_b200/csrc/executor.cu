@@ -287,7 +287,7 @@ __device__ __forceinline__ void emulated_task(const ReqDesc &d, const Task &t, i
         }
         case kPair:
             for (int64_t c = t.first; c < t.first + t.count; ++c)
-                oz::pair_chunk_body<T>(d.pair, c, tid, reinterpret_cast<double *>(work));
+                oz::pair_chunk_body<T>(d.pair, c, tid, reinterpret_cast<__nv_bfloat16 *>(work));
             break;
         case kSlice: {
             const oz::View &v = side ? d.vb : d.va;
@@ -849,8 +849,8 @@ int prepare(Executor *e, int slot, const Gemm &g, bool emulated, int mode, void 
         d.zero_ptr = reinterpret_cast<uint32_t *>(pt.err);
         d.zero_words = int64_t((reinterpret_cast<char *>(pt.ea) - reinterpret_cast<char *>(pt.err)) / 4);
         if (mode == 0 && d.forced == 0)  // (no chunks otherwise)
-            d.pair = oz::pair_sample(d.va, d.akc, d.vb, d.bkc, g.uplo, g.diag, 64, pt.pair);
-        Stage zero, stats, decide, slice, residue, recon;
+            d.pair = oz::pair_sample(d.va, d.akc, d.sa, d.vb, d.bkc, d.sbd, g.uplo, g.diag, 128, pt.pair);
+        Stage zero, stats, pair, decide, slice, residue, recon;
         add_tasks(zero, kZero, slot, 0, d.zero_words, spread(d.zero_words, 1 << 14, e->num_sms));
         for (int side = 0; side < (pl.alias ? 1 : 2); ++side) {
             const int64_t R = side ? pl.N : pl.M;
@@ -868,7 +868,7 @@ int prepare(Executor *e, int slot, const Gemm &g, bool emulated, int mode, void 
             const int64_t blocks = d.slice_gx[side] * (Rp / 64);
             add_tasks(slice, kSlice, slot, side, blocks, spread(blocks, 1, e->num_sms));
         }
-        add_tasks(stats, kPair, slot, 0, d.pair.chunks, 1);
+        add_tasks(pair, kPair, slot, 0, d.pair.chunks, 1);  // (takes the rows' norms from the statistics)
         add_tasks(decide, kDecide, slot, 0, 1, 1);
         d.res_tiles_j = pl.Jx / oz::kTileJ;
         d.res_tiles_i = pl.Ip / oz::kTileI;
@@ -882,7 +882,8 @@ int prepare(Executor *e, int slot, const Gemm &g, bool emulated, int mode, void 
         d.recon_gx = cdiv(pl.M, 512);
         add_tasks(recon, kRecon, slot, 0, d.recon_gx * pl.N, spread(d.recon_gx * pl.N, 8, e->num_sms));
         sl.stages = {zero, stats, decide, slice, residue, recon};
-        sl.decide_stage = 2;
+        if (d.pair.chunks) sl.stages.insert(sl.stages.begin() + 2, pair);
+        sl.decide_stage = int(sl.stages.size()) - 4;
         sl.fallback.push_back(native_stage(d, g, slot));
         sl.path = 2;
     }

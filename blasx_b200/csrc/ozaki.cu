@@ -36,10 +36,10 @@ namespace {
 template <typename T, int ROLE>
 __global__ void __launch_bounds__(256, ROLE == 0 ? 4 : (ROLE == 1 ? 3 : 2)) slice_kc_kernel(View v, RowStats st, const Decision *dec, int *expo,
                                                        SliceOut o, const __grid_constant__ PairVeto pv) {
-    __shared__ double2 smem[kPairShared / 2];
+    __shared__ __align__(16) __nv_bfloat16 smem[kPairShared];
     const int row0 = pv.p.chunks ? 1 : 0;
     if (blockIdx.y < row0) {
-        if (int(blockIdx.x) < pv.p.chunks) pair_veto_block<T>(pv, blockIdx.x, threadIdx.x, reinterpret_cast<double *>(smem));
+        if (int(blockIdx.x) < pv.p.chunks) pair_veto_block<T>(pv, blockIdx.x, threadIdx.x, smem);
         return;
     }
     slice_kc_body<T, ROLE>(v, st, dec, expo, o, blockIdx.x, blockIdx.y - row0, threadIdx.x);
@@ -49,10 +49,10 @@ template <typename T, int ROLE>
 __global__ void __launch_bounds__(256, ROLE == 0 ? 4 : (ROLE == 1 ? 3 : 2)) slice_rc_kernel(View v, RowStats st, const Decision *dec, int *expo,
                                                        SliceOut o, const __grid_constant__ PairVeto pv) {
     __shared__ __align__(16) unsigned char smem[slice_rc_smem_bytes<ROLE>()];
-    static_assert(sizeof smem >= kPairShared * sizeof(double), "the pair sample's stage");
+    static_assert(sizeof smem >= kPairShared * sizeof(__nv_bfloat16), "the pair sample's stage");
     const int row0 = pv.p.chunks ? 1 : 0;
     if (blockIdx.y < row0) {
-        if (int(blockIdx.x) < pv.p.chunks) pair_veto_block<T>(pv, blockIdx.x, threadIdx.x, reinterpret_cast<double *>(smem));
+        if (int(blockIdx.x) < pv.p.chunks) pair_veto_block<T>(pv, blockIdx.x, threadIdx.x, smem);
         return;
     }
     slice_rc_body<T, ROLE>(v, st, dec, expo, o, blockIdx.x, blockIdx.y - row0, threadIdx.x, smem);
@@ -70,10 +70,10 @@ struct SliceSide {
 template <typename T, bool AKC, bool BKC>
 __global__ void __launch_bounds__(256, 4) slice_both_kernel(SliceSide a, SliceSide b, int na, const Decision *dec,
                                                             const __grid_constant__ PairVeto pv) {
-    __shared__ __align__(16) unsigned char smem[(AKC && BKC) ? kPairShared * sizeof(double) : slice_rc_smem_bytes<0>()];
+    __shared__ __align__(16) unsigned char smem[(AKC && BKC) ? kPairShared * sizeof(__nv_bfloat16) : slice_rc_smem_bytes<0>()];
     const int i = int(blockIdx.x) - pv.p.chunks;
     if (i < 0) {
-        pair_veto_block<T>(pv, blockIdx.x, threadIdx.x, reinterpret_cast<double *>(smem));
+        pair_veto_block<T>(pv, blockIdx.x, threadIdx.x, smem);
     } else if (i < na) {
         if (AKC) slice_kc_body<T, 0>(a.v, a.st, dec, a.expo, a.o, i % a.gx, i / a.gx, threadIdx.x);
         else slice_rc_body<T, 0>(a.v, a.st, dec, a.expo, a.o, i % a.gx, i / a.gx, threadIdx.x, smem);
@@ -245,7 +245,8 @@ int ozaki_run(const Gemm &g, cudaStream_t s, int mode, void *ws, int num_sms, vo
     // of op(A)'s groups, one for eight rows, end before them.
     oz::PairVeto none{}, pv{};
     if (mode == 0 && oz::forced_moduli() == 0)
-        pv = oz::pair_veto(va, akc, vb, bkc, g.uplo, g.diag, pt, sb.flags - oz::kPairCounters, dec);
+        pv = oz::pair_veto(va, akc, sa, vb, bkc, pl.alias ? sa : sb, g.uplo, g.diag, pt,
+                           sb.flags - oz::kPairCounters, dec);
     const bool pv_first = pl.alias || oy.Rp <= ox.Rp;
     if constexpr (CPLX) {
         BX_TRY((launch_slice<T, 1>(va, akc, sa, dec, ea, oy, Kc, pv_first ? pv : none, s)));

@@ -16,6 +16,8 @@
 #include <cstring>
 #include <type_traits>
 
+#include <cuda_bf16.h>
+
 #include "ozaki.h"
 
 namespace bx {
@@ -226,30 +228,37 @@ __device__ __forceinline__ void stats_rc_body(const View &v, const RowStats &st,
 //   n = sum_k |a_ik| |b_kj| / (||a_i||_2 ||b_j||_2)
 // over their pairs inside the output's triangle enters the estimate. Pairs
 // whose sum is zero have an exact zero in C and do not count.
-// What bounds it: latency (a few thousand scattered loads). So the k extent is
-// cut into chunks of kPairChunk, a block of 256 threads each with all loads of
-// a step in flight; the chunks' partial sums go to scratch and are added in
-// chunk order. The standalone path runs these blocks among those of the slices,
-// which hide them (PairVeto, ozaki_stats.cuh).
-constexpr int kPairRows = 32, kPairStep = 32, kPairChunk = 64;
-constexpr int kPairLd = kPairRows + 2;                            // row of a staged k
-constexpr int kPairShared = 2 * kPairStep * kPairLd;              // doubles
-constexpr int kPairPart = kPairRows * kPairRows + 2 * kPairRows;  // doubles per chunk: products, then sums of squares
+// What bounds it: the chain of a load, a hand-over and a sum, with few issue
+// slots beside the slices' blocks (PairVeto, ozaki_stats.cuh). So the k extent
+// is cut into chunks of kPairChunk, a block of 256 threads each with all loads
+// of a step in flight, and the products run as bf16 MMAs on rows scaled by
+// their norms, one 16 x 8 tile of pairs per warp; the chunks' FP32 sums go to
+// scratch and are added in chunk order. (In FP64 on the CUDA cores, with the
+// norms from the sample itself, a chunk took 17 to 26 thousand cycles beside
+// the slices and the sum of 16 chunks 18; now 14 to 24 and 9, and DSYRK 4000 x
+// 1000, whose slices are short, 279 us against 276 without the sample and now.)
+constexpr int kPairRows = 32, kPairChunk = 64;
+constexpr int kPairLd = kPairChunk + 8;                 // row of a staged step, conflict-free fragment reads
+constexpr int kPairShared = 2 * kPairRows * kPairLd;    // bf16
+constexpr int kPairPart = kPairRows * kPairRows;        // floats per chunk: thread t holds pairs 4 t .. 4 t + 3
 struct PairSample {
     View v[2];       // op(A) rows, op(B) columns over k
+    const double *sumsq[2];
     int kc[2];       // k-contiguous source
     int uplo;
     int64_t diag;
     int chunks;
     int64_t kchunk;
-    double *part;    // [chunks][kPairPart]
+    float *part;     // [chunks][kPairPart]
 };
 
-inline PairSample pair_sample(const View &va, bool akc, const View &vb, bool bkc, int uplo, int64_t diag,
-                              int max_chunks, double *part) {
+inline PairSample pair_sample(const View &va, bool akc, const RowStats &sa, const View &vb, bool bkc,
+                              const RowStats &sb, int uplo, int64_t diag, int max_chunks, float *part) {
     PairSample p;
     p.v[0] = va;
     p.v[1] = vb;
+    p.sumsq[0] = sa.sumsq;
+    p.sumsq[1] = sb.sumsq;
     p.kc[0] = akc;
     p.kc[1] = bkc;
     p.uplo = uplo;
@@ -268,87 +277,94 @@ __device__ __forceinline__ int64_t pair_row(int s, int64_t R, int side) {
     return lo + ((hi - lo) * ((s * 20 + 7 + 11 * side) % kPairRows)) / kPairRows;
 }
 
-// One chunk, by 256 threads; sh: kPairShared doubles.
+// The (row, column) of value r of a thread's four: the accumulator layout of
+// mma.m16n8k16, warp w holding rows 16 (w % 2) .. and columns 8 (w / 2) ..
+__device__ __forceinline__ int pair_i(int tid, int r) {
+    return 16 * (tid >> 5 & 1) + (tid & 31) / 4 + (r >= 2 ? 8 : 0);
+}
+__device__ __forceinline__ int pair_j(int tid, int r) { return 8 * (tid >> 6) + 2 * (tid & 3) + (r & 1); }
+
+// One chunk, by 256 threads; sh: kPairShared bf16.
 template <typename T>
-__device__ __forceinline__ void pair_chunk_body(const PairSample &p, int64_t chunk, int tid, double *sh) {
+__device__ __forceinline__ void pair_chunk_body(const PairSample &p, int64_t chunk, int tid, __nv_bfloat16 *sh) {
     const int64_t k0 = chunk * p.kchunk, k1 = min(p.v[0].K, k0 + p.kchunk);
-    const int lane = tid & 31, warp = tid >> 5;        // a warp loads rows warp, warp + 8, ... of both operands
-    const int i = 2 * (tid / 16), j = 2 * (tid % 16);  // this thread's 2 x 2 pairs
-    double ssq[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}}, sum[2][2] = {{0, 0}, {0, 0}};
-    for (int64_t k = k0; k < k1; k += kPairStep) {
+    const int lane = tid & 31, warp = tid >> 5;  // a warp loads rows warp, warp + 8, ... of both operands
+    // lane 4 side + h: the reciprocal norm of row warp + 8 h
+    double inv = 0.0;
+    if (lane < 8) {
+        const int sd = lane >> 2;
+        const double q = p.sumsq[sd][pair_row(warp + 8 * (lane & 3), p.v[sd].R, sd)];
+        if (q > 0) inv = 1.0 / sqrt(q);
+    }
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int64_t k = k0; k < k1; k += kPairChunk) {
         __syncthreads();  // the last step has been read
 #pragma unroll
         for (int sd = 0; sd < 2; ++sd)
 #pragma unroll
             for (int h = 0; h < 4; ++h) {
-                double x = 0.0, y = 0.0;
-                if (k + lane < k1)
-                    load_elem<T>(p.v[sd], pair_row(warp + 8 * h, p.v[sd].R, sd), k + lane, p.kc[sd] != 0, x, y);
-                ssq[sd][h] = fma(x, x, fma(y, y, ssq[sd][h]));
-                sh[(sd * kPairStep + lane) * kPairLd + warp + 8 * h] = fabs(x) + fabs(y);
+                const int64_t row = pair_row(warp + 8 * h, p.v[sd].R, sd);
+                const double scale = __shfl_sync(0xffffffffu, inv, 4 * sd + h);
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const int64_t kk = k + lane + 32 * u;
+                    double x = 0.0, y = 0.0;
+                    if (kk < k1) load_elem<T>(p.v[sd], row, kk, p.kc[sd] != 0, x, y);
+                    const double m = fabs(x) + fabs(y);
+                    // (no product of two nonzero entries vanishes)
+                    const float f = m > 0 ? fmaxf(float(m * scale), 1e-18f) : 0.f;
+                    sh[(sd * kPairRows + warp + 8 * h) * kPairLd + lane + 32 * u] = __float2bfloat16_rn(f);
+                }
             }
         __syncthreads();
-#pragma unroll 8
-        for (int q = 0; q < kPairStep; ++q) {
-            const double2 a = *reinterpret_cast<const double2 *>(&sh[q * kPairLd + i]);
-            const double2 b = *reinterpret_cast<const double2 *>(&sh[(kPairStep + q) * kPairLd + j]);
-            sum[0][0] = fma(a.x, b.x, sum[0][0]);
-            sum[0][1] = fma(a.x, b.y, sum[0][1]);
-            sum[1][0] = fma(a.y, b.x, sum[1][0]);
-            sum[1][1] = fma(a.y, b.y, sum[1][1]);
-        }
+        const uint32_t *a = reinterpret_cast<const uint32_t *>(
+            sh + (16 * (warp & 1) + lane / 4) * kPairLd + 2 * (lane & 3));
+        const uint32_t *b = reinterpret_cast<const uint32_t *>(
+            sh + (kPairRows + 8 * (warp >> 1) + lane / 4) * kPairLd + 2 * (lane & 3));
+#pragma unroll
+        for (int q = 0; q < kPairChunk / 16; ++q)
+            asm volatile(
+                "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                : "+f"(acc[0]), "+f"(acc[1]), "+f"(acc[2]), "+f"(acc[3])
+                : "r"(a[8 * q]), "r"(a[8 * q + 4 * kPairLd]), "r"(a[8 * q + 4]), "r"(a[8 * q + 4 + 4 * kPairLd]),
+                  "r"(b[8 * q]), "r"(b[8 * q + 4]));
     }
-    double *w = p.part + chunk * kPairPart;
-#pragma unroll
-    for (int a = 0; a < 2; ++a)
-#pragma unroll
-        for (int b = 0; b < 2; ++b) w[(i + a) * kPairRows + j + b] = sum[a][b];
-#pragma unroll
-    for (int sd = 0; sd < 2; ++sd)
-#pragma unroll
-        for (int h = 0; h < 4; ++h) {
-            double v = ssq[sd][h];
-            for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == 0) w[kPairRows * kPairRows + sd * kPairRows + warp + 8 * h] = v;
-        }
+    reinterpret_cast<float4 *>(p.part + chunk * kPairPart)[tid] = make_float4(acc[0], acc[1], acc[2], acc[3]);
 }
 
-// The sum of n partial results: this thread's values e = tid, tid + 256, ...
-constexpr int kPairPer = (kPairPart + 255) / 256;
-__device__ __forceinline__ void pair_add(const double *in, int n, int tid, double (&v)[kPairPer]) {
-#pragma unroll
-    for (int q = 0; q < kPairPer; ++q) v[q] = 0;
-#pragma unroll 4
-    for (int c = 0; c < n; ++c, in += kPairPart)
-#pragma unroll
-        for (int q = 0; q < kPairPer; ++q) {
-            const int e = tid + 256 * q;
-            if (e < kPairPart) v[q] += __ldcg(in + e);
-        }
+// The sum of n partial results: this thread's four pairs.
+__device__ __forceinline__ float4 pair_add(const float *in, int n, int tid) {
+    const float4 *p = reinterpret_cast<const float4 *>(in) + tid;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (int c = 0; c < n; ++c, p += kPairPart / 4) {
+        const float4 x = __ldcg(p);
+        v.x += x.x;
+        v.y += x.y;
+        v.z += x.z;
+        v.w += x.w;
+    }
+    return v;
 }
 
 // The smallest n over the pairs from `count` partial results at `in` (256
-// threads; the result is in thread 0). 1e300 when no pair counts.
-__device__ __forceinline__ double pair_reduce(const PairSample &p, const double *in, int count, int tid, double *sh) {
-    static_assert(kPairRows * kPairRows % 256 == 0 && 2 * kPairRows <= 256, "a thread's last value is a sum of squares");
-    double v[kPairPer];
-    pair_add(in, count, tid, v);
-    __syncthreads();  // sh is free
-    if (tid < 2 * kPairRows) sh[tid] = sqrt(v[kPairPer - 1]);
-    __syncthreads();
-    double least = 1e300;
+// threads; the result is in thread 0; sh: 8 floats). 1e30 when no pair counts.
+__device__ __forceinline__ float pair_reduce(const PairSample &p, const float *in, int count, int tid, float *sh) {
+    const float4 s = pair_add(in, count, tid);
+    const float v[4] = {s.x, s.y, s.z, s.w};
+    float least = 1e30f;
 #pragma unroll
-    for (int q = 0; q < kPairPer - 1; ++q) {
-        const int e = tid + 256 * q, i = e / kPairRows, j = e % kPairRows;
-        const int64_t d = pair_row(i, p.v[0].R, 0) - pair_row(j, p.v[1].R, 1);
+    for (int r = 0; r < 4; ++r) {
+        const int64_t d = pair_row(pair_i(tid, r), p.v[0].R, 0) - pair_row(pair_j(tid, r), p.v[1].R, 1);
         if (p.uplo && (p.uplo == 1 ? d > p.diag : d < p.diag)) continue;
-        if (v[q] > 0) least = fmin(least, v[q] / (sh[i] * sh[kPairRows + j]));
+        if (v[r] > 0.f) least = fminf(least, v[r]);
     }
-    for (int o = 16; o; o >>= 1) least = fmin(least, __shfl_xor_sync(0xffffffffu, least, o));
-    if (tid % 32 == 0) sh[2 * kPairRows + tid / 32] = least;
+    for (int o = 16; o; o >>= 1) least = fminf(least, __shfl_xor_sync(0xffffffffu, least, o));
+    __syncthreads();  // sh is free
+    if (tid % 32 == 0) sh[tid / 32] = least;
     __syncthreads();
     if (tid == 0)
-        for (int w = 1; w < 8; ++w) least = fmin(least, sh[2 * kPairRows + w]);
+        for (int w = 1; w < 8; ++w) least = fminf(least, sh[w]);
     return least;
 }
 
@@ -373,9 +389,10 @@ __device__ __forceinline__ double paired_estimate(double est, double spread, dou
 __device__ __forceinline__ void decide_body(const RowStats &sa, int64_t Ra, const RowStats &sb, int64_t Rb,
                                            int64_t K, double unit, int mode, int forced, Decision *dec,
                                            const PairSample &ps, int tid, int nthreads) {
-    __shared__ double s_rho[2][32], s_h[2][32], s_pair[2 * kPairRows + 8];
+    __shared__ double s_rho[2][32], s_h[2][32];
+    __shared__ float s_pair[8];
     __shared__ int s_bad[32];
-    const double least = ps.chunks ? pair_reduce(ps, ps.part, ps.chunks, tid, s_pair) : 1e300;
+    const double least = ps.chunks ? pair_reduce(ps, ps.part, ps.chunks, tid, s_pair) : 1e30;
     double rho[2] = {0, 0}, h[2] = {1e300, 1e300};
     int bad = 0;
     for (int side = 0; side < 2; ++side) {
@@ -1234,7 +1251,7 @@ struct Parts {
     int *ea, *fb;
     int8_t *Y, *X;
     uint8_t *U;
-    double *pair;  // partial results of the pair sample
+    float *pair;  // partial results of the pair sample
     int64_t pair_slots;  // and how many there is room for
 };
 inline Parts carve_parts(const Gemm &g, const Plan &pl, void *ws) {
@@ -1254,10 +1271,10 @@ inline Parts carve_parts(const Gemm &g, const Plan &pl, void *ws) {
     p.X = pl.alias ? p.Y : cv.take<int8_t>(size_t(L) * pl.Jx * pl.Kp);
     p.U = cv.take<uint8_t>(size_t(L) * pl.Jx * pl.Ip);
     // in U, which the residue GEMM is the first to write
-    p.pair = reinterpret_cast<double *>(p.U);
-    p.pair_slots = int64_t(L) * pl.Jx * pl.Ip / int64_t(kPairPart * sizeof(double));
-    static_assert(int64_t(kMaxModuli) * kTileJ * kTileI / int64_t(kPairPart * sizeof(double)) >= 64 + 8 + 1,
-                  "64 chunks, their groups and the result fit the smallest U");
+    p.pair = reinterpret_cast<float *>(p.U);
+    p.pair_slots = int64_t(L) * pl.Jx * pl.Ip / int64_t(kPairPart * sizeof(float));
+    static_assert(int64_t(kMaxModuli) * kTileJ * kTileI / int64_t(kPairPart * sizeof(float)) >= 128 + 12 + 1,
+                  "128 chunks, their groups and the result fit the smallest U");
     return p;
 }
 

@@ -348,10 +348,8 @@ template <typename T> __global__ void __launch_bounds__(kStatsThreads) stats_dec
 // large entries do not meet. (Decision::slices keeps the count for the slices
 // that run meanwhile.) As part of the statistics the sample's chain of loads
 // and hand-overs delayed the decision: 7.6 us at FP64 2048^3, 10.3 at FP32
-// 3001 x 1777 x 999. Beside the slices it costs less than 1 us there, and 6 us
-// where they are shorter than its chain (DSYRK 4000 x 1000: 22.6 -> 28.5). The
-// chunks are added in two levels, groups of 16 or the square root of their
-// number.
+// 3001 x 1777 x 999. Beside the slices it costs about 1 us there. The chunks are
+// added in two levels, groups of 16 or the square root of their number.
 constexpr int kPairMaxGroup = 32, kPairCounters = kPairMaxGroup + 1;
 struct PairVeto {
     PairSample p;  // no chunks: no sample
@@ -360,13 +358,13 @@ struct PairVeto {
     Decision *dec;
 };
 // counters: kPairCounters words.
-inline PairVeto pair_veto(const View &va, bool akc, const View &vb, bool bkc, int uplo, int64_t diag,
-                          const Parts &pt, int *counters, Decision *dec) {
+inline PairVeto pair_veto(const View &va, bool akc, const RowStats &sa, const View &vb, bool bkc, const RowStats &sb,
+                          int uplo, int64_t diag, const Parts &pt, int *counters, Decision *dec) {
     PairVeto a;
-    // (64 chunks fit the smallest scratch; slots for the groups and the result)
-    const int64_t room = std::max<int64_t>(64, pt.pair_slots - kPairCounters - 1);
-    a.p = pair_sample(va, akc, vb, bkc, uplo, diag, int(std::min<int64_t>(room, kPairMaxGroup * kPairMaxGroup)),
-                      pt.pair);
+    // (128 chunks fit the smallest scratch; slots for the groups and the result)
+    const int64_t room = std::max<int64_t>(128, pt.pair_slots - kPairCounters - 1);
+    a.p = pair_sample(va, akc, sa, vb, bkc, sb, uplo, diag,
+                      int(std::min<int64_t>(room, kPairMaxGroup * kPairMaxGroup)), pt.pair);
     a.group = 16;
     while (a.group * a.group < a.p.chunks) ++a.group;
     a.arrive = counters;
@@ -388,23 +386,24 @@ __device__ __forceinline__ bool last_arrival(int *counter, int of, int tid) {
 }
 
 template <typename T>
-__device__ __noinline__ void pair_veto_block(const PairVeto &a, int chunk, int tid, double *sh) {
+__device__ __noinline__ void pair_veto_block(const PairVeto &a, int chunk, int tid, void *sh) {
     const PairSample &p = a.p;
     if (a.dec->slices == 0) return;  // native already
     const int per = a.group, groups = (p.chunks + per - 1) / per, group = chunk / per;
-    double *sums = p.part + int64_t(p.chunks) * kPairPart;
-    pair_chunk_body<T>(p, chunk, tid, sh);
     const int n = min(per, p.chunks - group * per);
+    float *sums = p.part + int64_t(p.chunks) * kPairPart;
+    pair_chunk_body<T>(p, chunk, tid, static_cast<__nv_bfloat16 *>(sh));
     if (!last_arrival(a.arrive + group, n, tid)) return;
+    const float *in = p.part;
+    int count = n;
     if (groups > 1) {
-        double v[kPairPer];
-        pair_add(p.part + int64_t(group) * per * kPairPart, n, tid, v);
-#pragma unroll
-        for (int q = 0; q < kPairPer; ++q)
-            if (tid + 256 * q < kPairPart) sums[int64_t(group) * kPairPart + tid + 256 * q] = v[q];
+        reinterpret_cast<float4 *>(sums + int64_t(group) * kPairPart)[tid] =
+            pair_add(p.part + int64_t(group) * per * kPairPart, n, tid);
         if (!last_arrival(a.arrive + kPairMaxGroup, groups, tid)) return;
+        in = sums;
+        count = groups;
     }
-    const double least = groups > 1 ? pair_reduce(p, sums, groups, tid, sh) : pair_reduce(p, p.part, n, tid, sh);
+    const float least = pair_reduce(p, in, count, tid, static_cast<float *>(sh));
     if (tid == 0) {
         const double est = paired_estimate(a.dec->estimate, a.dec->spread, least);
         a.dec->estimate = est;
