@@ -167,26 +167,28 @@ constexpr TileModel kCplx[] = {{1, 64, 64, 2, {0.72, 0.86, 0, 0}}, {2, 32, 32, 4
 // at a time (as DmmaParams::vec_a).
 bool wide_copies(const void *p, int64_t ld) { return ld % 2 == 0 && reinterpret_cast<uintptr_t>(p) % 16 == 0; }
 
-// What a tile loses against its fraction on some layouts of the operands, with
-// n CTAs of it per SM.
+// What a tile loses against its fraction on some layouts of the operands, in
+// full rounds (n = 0) or in the last one with n CTAs of it per SM.
 // Two k-contiguous operands: 32x32 FP64 tiles 15%, 64x64 complex128 tiles 20%
 // (3000 x 3000 x 200: 634 us, 520 with 32x32 tiles; 2496 x 3072 x 83: 296 and
 // 230; the 64x128 tile, which served them before, 583 and 270).
 // FP64 operands that are m- or n-contiguous and copied 8 bytes at a time (odd
 // leading dimension): a smaller tile copies more of them per multiply-add, 6%
 // each against 64x64 (1000^3 NT: 32x32 tiles 111 us, 64x64 95; with even ones
-// 89 and 85).
+// 89 and 85), which lose 5% with three per SM in the last round (9832 x 116 x
+// 721 NN, odd: 105 us, 32x32 93).
 // 64x48 tiles of two such operands (NT) cover their latencies badly with one
 // or two CTAs per SM, whatever the copies (1003 x 777 x 641, odd: 70.5 us,
 // 64x64 64.2).
 double layout_cost(const TileModel &m, double macs, const Gemm &g, int64_t n) {
     const bool a_k = g.ta != NoTrans, b_k = g.tb == NoTrans;
     if (macs != 1.0) return m.g == 1 && a_k && b_k ? 1.2 : 1.0;
-    if (m.g != 2 && m.g != 3) return 1.0;
     const int narrow = (!a_k && !wide_copies(g.A, g.lda)) + (!b_k && !wide_copies(g.B, g.ldb));
+    if (m.g == 1) return narrow && n == 3 ? 1.05 : 1.0;
+    if (m.g == 0) return 1.0;
     double cost = 1.0 + (m.g == 2 ? 0.06 : 0.065) * narrow;
     if (m.g == 2 && a_k && b_k) cost *= 1.15;
-    if (m.g == 3 && !a_k && !b_k && n <= 2) cost *= 1.12;
+    if (m.g == 3 && !a_k && !b_k && (n == 1 || n == 2)) cost *= 1.12;
     return cost;
 }
 
@@ -202,7 +204,7 @@ template <int COUNT> Geometry pick_geometry(const TileModel (&models)[COUNT], do
             const int64_t ctas = tiles * s, round = sms * m.per_sm, rest = ctas % round;
             const int64_t n = (rest + sms - 1) / sms;
             const double share = macs * m.bm * m.bn * double((g.K + s - 1) / s) / 64.0;
-            const double t = share * (layout_cost(m, macs, g, m.per_sm) * double(ctas / round) * m.per_sm /
+            const double t = share * (layout_cost(m, macs, g, 0) * double(ctas / round) * m.per_sm /
                                           m.eff[m.per_sm - 1] +
                                       (n ? layout_cost(m, macs, g, n) * double(n) / m.eff[n - 1] : 0.0)) +
                              (s > 1 ? kSplitCycles : 0.0);
