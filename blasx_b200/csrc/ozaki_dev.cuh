@@ -234,9 +234,8 @@ __device__ __forceinline__ void stats_rc_body(const View &v, const RowStats &st,
 // of a step in flight, and the products run as bf16 MMAs on rows scaled by
 // their norms, one 16 x 8 tile of pairs per warp; the chunks' FP32 sums go to
 // scratch and are added in chunk order. (In FP64 on the CUDA cores, with the
-// norms from the sample itself, a chunk took 17 to 26 thousand cycles beside
-// the slices and the sum of 16 chunks 18; now 14 to 24 and 9, and DSYRK 4000 x
-// 1000, whose slices are short, 279 us against 276 without the sample and now.)
+// norms from the sample itself, a chunk took 17 to 34 thousand cycles beside
+// the slices and the sum of 16 chunks 18; now 8 to 21 and 7.)
 constexpr int kPairRows = 32, kPairChunk = 64;
 constexpr int kPairLd = kPairChunk + 8;                 // row of a staged step, conflict-free fragment reads
 constexpr int kPairShared = 2 * kPairRows * kPairLd;    // bf16
@@ -289,28 +288,42 @@ template <typename T>
 __device__ __forceinline__ void pair_chunk_body(const PairSample &p, int64_t chunk, int tid, __nv_bfloat16 *sh) {
     const int64_t k0 = chunk * p.kchunk, k1 = min(p.v[0].K, k0 + p.kchunk);
     const int lane = tid & 31, warp = tid >> 5;  // a warp loads rows warp, warp + 8, ... of both operands
-    // lane 4 side + h: the reciprocal norm of row warp + 8 h
+    using R = typename Elem<T>::R;
+    constexpr int PER = Elem<T>::cplx ? 2 : 1;
+    // lane 4 side + h: the norm of row warp + 8 h, on its way with the first step
     double inv = 0.0;
-    if (lane < 8) {
-        const int sd = lane >> 2;
-        const double q = p.sumsq[sd][pair_row(warp + 8 * (lane & 3), p.v[sd].R, sd)];
-        if (q > 0) inv = 1.0 / sqrt(q);
-    }
+    if (lane < 8) inv = p.sumsq[lane >> 2][pair_row(warp + 8 * (lane & 3), p.v[lane >> 2].R, lane >> 2)];
+    bool first = true;
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
     for (int64_t k = k0; k < k1; k += kPairChunk) {
-        __syncthreads();  // the last step has been read
+        R e[2][4][2][PER];
 #pragma unroll
         for (int sd = 0; sd < 2; ++sd)
 #pragma unroll
             for (int h = 0; h < 4; ++h) {
                 const int64_t row = pair_row(warp + 8 * h, p.v[sd].R, sd);
-                const double scale = __shfl_sync(0xffffffffu, inv, 4 * sd + h);
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
                     const int64_t kk = k + lane + 32 * u;
-                    double x = 0.0, y = 0.0;
-                    if (kk < k1) load_elem<T>(p.v[sd], row, kk, p.kc[sd] != 0, x, y);
-                    const double m = fabs(x) + fabs(y);
+                    const R *q = static_cast<const R *>(p.v[sd].p) +
+                                 PER * (p.kc[sd] ? kk + row * p.v[sd].ld : row + kk * p.v[sd].ld);
+#pragma unroll
+                    for (int c = 0; c < PER; ++c) e[sd][h][u][c] = kk < k1 ? q[c] : R(0);
+                }
+            }
+        if (first) inv = inv > 0 ? 1.0 / sqrt(inv) : 0.0;
+        first = false;
+        __syncthreads();  // the last step has been read
+#pragma unroll
+        for (int sd = 0; sd < 2; ++sd)
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                const double scale = __shfl_sync(0xffffffffu, inv, 4 * sd + h);
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    double m = 0.0;
+#pragma unroll
+                    for (int c = 0; c < PER; ++c) m += fabs(double(e[sd][h][u][c]));
                     // (no product of two nonzero entries vanishes)
                     const float f = m > 0 ? fmaxf(float(m * scale), 1e-18f) : 0.f;
                     sh[(sd * kPairRows + warp + 8 * h) * kPairLd + lane + 32 * u] = __float2bfloat16_rn(f);
