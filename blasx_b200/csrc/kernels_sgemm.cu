@@ -27,7 +27,8 @@ bool narrow_copies(const void *p, int64_t ld) { return ld % 4 != 0 || reinterpre
 // it through registers, each element for 128 outputs. Measured, FMA / this one,
 // both operands narrow: 8000 x 8000 x 2000 NN 7.89 / 6.51 ms, NT 7.99 / 6.41;
 // 4000 x 4000 x 1000 NN 1042 / 881 us; 2500 x 2500 x 600 NT 272 / 241; 3000 x
-// 3000 x 256 NN 169 / 165, but 4000 x 4000 x 100 155 / 165. One of them: 8000 x
+// 3000 x 256 NN 169 / 165; 2100 x 2150 NT x 250 95 / 86, x 200 81 / 73, x 160 66
+// / 66, x 80 42 / 51; 4000 x 4000 x 100 155 / 165. One of them: 8000 x
 // 8000 x 2000 6.78 to 7.33 / 6.5, 3000 x 3000 x 1000 507 to 546 / 494, 8000 x
 // 4000 x 512 914 to 1006 / 950, 3000 x 3000 x 256 147 to 157 / 164. With 16-byte
 // copies FMA is as fast or faster everywhere. Two of these CTAs share an SM and
@@ -37,7 +38,7 @@ bool sgemm128_preferred(const Gemm &g) {
     using namespace dev::sg;
     if (g.dt != DType::F32 || g.M > INT32_MAX || g.N > INT32_MAX || g.K > INT32_MAX) return false;
     const int narrow = narrow_copies(g.A, g.lda) + narrow_copies(g.B, g.ldb);
-    if (narrow == 0 || g.K < (narrow == 2 ? 256 : 640)) return false;
+    if (narrow == 0 || g.K < (narrow == 2 ? 192 : 640)) return false;
     const int64_t tiles = ((g.M + TM - 1) / TM) * ((g.N + TN - 1) / TN);
     const int64_t small = ((g.M + 63) / 64) * ((g.N + 63) / 64);
     const int64_t rounds = (tiles + kSms - 1) / kSms;  // tiles of the busiest SM

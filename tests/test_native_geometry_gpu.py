@@ -103,7 +103,8 @@ def test_fp64_tiles_by_copy_width(native, ta, tb, shape, pad, tile):
 
 @pytest.mark.parametrize("ta,tb", [("N", "N"), ("N", "T"), ("T", "N"), ("T", "T")])
 @pytest.mark.parametrize("shape,pad,tile", [((2500, 2492, 300), 1, (128, 128)), ((2500, 2492, 300), 0, (64, 64)),
-                                            ((2170, 2165, 257), 0, (128, 128)), ((2500, 2492, 250), 1, (64, 64)),
+                                            ((2170, 2165, 257), 0, (128, 128)), ((2100, 2150, 192), 1, (128, 128)),
+                                            ((2100, 2150, 191), 1, (64, 64)),
                                             ((2400, 2400, 300), 1, (64, 64))])
 def test_fp32_tiles_by_copy_width(native, ta, tb, shape, pad, tile):
     m, n, k = shape
