@@ -33,16 +33,22 @@ bool narrow_copies(const void *p, int64_t ld) { return ld % 4 != 0 || reinterpre
 // 4000 x 512 914 to 1006 / 950, 3000 x 3000 x 256 147 to 157 / 164. With 16-byte
 // copies FMA is as fast or faster everywhere. Two of these CTAs share an SM and
 // a tile is four 64x64 ones: the last round's idle SMs count against it (2400 x
-// 2400 x 300, 361 tiles: 134 / 146; 4000 x 2000 x 700, 512: 390 / 360).
+// 2400 x 300, 361 tiles: 134 / 146; 4000 x 2000 x 700, 512: 390 / 360). These
+// read C (beta 0.5), which costs this tile's epilogue more than FMA's; with beta
+// = 0 its lines lie lower: both narrow 8000 x 4000 NT x 250 572 / 473 us, x 140
+// 354 / 302, x 96 260 / 232, x 64 193 / 184; one, x 400 725 to 791 / 700, x 200
+// 415 to 440 / 391, x 100 254 to 266 / 245, 4000 x 4000 x 64 90 to 96 / 98.
 bool sgemm128_preferred(const Gemm &g) {
     using namespace dev::sg;
     if (g.dt != DType::F32 || g.M > INT32_MAX || g.N > INT32_MAX || g.K > INT32_MAX) return false;
     const int narrow = narrow_copies(g.A, g.lda) + narrow_copies(g.B, g.ldb);
-    if (narrow == 0 || g.K < (narrow == 2 ? 192 : 640)) return false;
+    const bool reads_c = !g.beta_zero();
+    if (narrow == 0 || g.K < (reads_c ? (narrow == 2 ? 192 : 640) : 96)) return false;
+    const double area = narrow == 2 ? 1.19 : (reads_c ? 1.08 : 1.13);
     const int64_t tiles = ((g.M + TM - 1) / TM) * ((g.N + TN - 1) / TN);
     const int64_t small = ((g.M + 63) / 64) * ((g.N + 63) / 64);
     const int64_t rounds = (tiles + kSms - 1) / kSms;  // tiles of the busiest SM
-    return (g.N + TN - 1) / TN <= 65535 && double(rounds * kSms * 4) < (narrow == 2 ? 1.19 : 1.08) * double(small);
+    return (g.N + TN - 1) / TN <= 65535 && double(rounds * kSms * 4) < area * double(small);
 }
 
 int launch_sgemm128(const Gemm &g, cudaStream_t s) {

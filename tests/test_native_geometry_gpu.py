@@ -59,7 +59,7 @@ def op(x, t):
     return x.mT if t == "N" else (x.conj() if t == "C" else x)
 
 
-def run(blx, dt, ta, tb, m, n, k, pad, tile, cut):
+def run(blx, dt, ta, tb, m, n, k, pad, tile, cut, beta=-1.0):
     gen = torch.Generator(device="cuda")
     gen.manual_seed(m + n + k)
     top = 2 if dt in "sc" else 8  # sums below 2^24 (2^53)
@@ -69,7 +69,7 @@ def run(blx, dt, ta, tb, m, n, k, pad, tile, cut):
     out = C.clone()
 
     def call():
-        rc = blx.gemm_device(ta, tb, m, n, k, 2.0, A, ra + pad, B, rb + pad, -1.0, out, m + pad, dtype=dt)
+        rc = blx.gemm_device(ta, tb, m, n, k, 2.0, A, ra + pad, B, rb + pad, beta, out, m + pad, dtype=dt)
         assert rc == blx.BLASX_OK, blx.last_error()
 
     kernels = launched(call)
@@ -80,7 +80,7 @@ def run(blx, dt, ta, tb, m, n, k, pad, tile, cut):
     assert blocks == tiles * cut and ("split" in name) == (cut > 1), (name, blocks, tiles)
     wide = torch.complex128 if dt in "zc" else torch.float64
     want = C.to(wide).clone()
-    want[:, :m] = (2 * (op(A[:, :ra].to(wide), ta) @ op(B[:, :rb].to(wide), tb)) - C[:, :m].to(wide).mT).mT
+    want[:, :m] = (2 * (op(A[:, :ra].to(wide), ta) @ op(B[:, :rb].to(wide), tb)) + beta * C[:, :m].to(wide).mT).mT
     assert torch.equal(out.to(wide), want)
 
 
@@ -109,6 +109,15 @@ def test_fp64_tiles_by_copy_width(native, ta, tb, shape, pad, tile):
 def test_fp32_tiles_by_copy_width(native, ta, tb, shape, pad, tile):
     m, n, k = shape
     run(native, "s", ta, tb, m, n, k, pad, tile, 1)
+
+
+@pytest.mark.parametrize("ta,tb,shape,pad,tile", [
+    ("N", "N", (2100, 2150, 96), 1, (128, 128)), ("T", "N", (2100, 2150, 95), 1, (64, 64)),
+    ("N", "T", (2100, 2150, 96), 0, (128, 128)), ("N", "T", (2100, 2150, 95), 0, (64, 64)),  # op(B) alone narrow
+    ("N", "N", (2100, 2152, 300), 0, (64, 64)),
+])
+def test_fp32_tiles_without_c(native, ta, tb, shape, pad, tile):
+    run(native, "s", ta, tb, *shape, pad, tile, 1, beta=0.0)
 
 
 def test_fp32_large_tile_as_the_fallback(blx):
