@@ -1,5 +1,5 @@
 // fma_tile.cuh -- the native FP32 / complex64 GEMM tile on the CUDA cores of
-// the standalone kernel (kernels_simt.cu).
+// the standalone kernels (kernels_fma.cu).
 //
 // What bounds a small product is not arithmetic: it is how many SMs get a
 // tile and how long a tile's chain of loads is. So the tiles are small (32x32

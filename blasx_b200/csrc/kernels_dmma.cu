@@ -32,10 +32,11 @@ __global__ void __launch_bounds__(Tile<CPLX, G>::THREADS, Tile<CPLX, G>::PER_SM)
 
 // The emulated path's fallback: one resident set of CTAs that take tiles from
 // a counter. It usually has nothing to do, and the exits of a CTA per tile took
-// 6 us at 2048^3. (From four sets of tiles on it is a CTA per tile again: the
-// counter costs a product that does fall back 2.6%, 4096 x 3000 x 2500, tiles
-// dealt out in advance 6%, and the exits cost a large product less. A kernel
-// of its own: the loop in the plain one made that 3% slower.)
+// 6 us at 2048^3. A product that does fall back pays for the counter: 653 us
+// there, 559 with a CTA per tile. (From four sets of tiles on it is a CTA per
+// tile again: the counter cost 4096 x 3000 x 2500 2.6%, tiles dealt out in
+// advance 6%, and the exits cost a large product less. A kernel of its own: the
+// loop in the plain one made that 3% slower.)
 template <bool CPLX, bool AKC, bool BKC, int KI, int G>
 __global__ void __launch_bounds__(Tile<CPLX, G>::THREADS, Tile<CPLX, G>::PER_SM)
     dmma_queue_kernel(const DmmaParams p) {

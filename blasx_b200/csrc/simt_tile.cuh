@@ -116,8 +116,9 @@ __device__ __forceinline__ void simt_tile(const SimtParams<T> &p, int64_t bm, in
 
 // ---- FP32 on the CUDA cores, 128 x 128 C tile per CTA of 256 threads ----------
 //
-// The serving executor's FP32 tile (standalone calls: fma_tile.cuh, as fast at
-// 4096 x 4096 x 1024, faster below).
+// The serving executor's FP32 tile, and that of large standalone products whose
+// operands cannot be copied 16 bytes at a time (kernels_sgemm.cu; the others:
+// fma_tile.cuh).
 // The 64 x 64 tile above computes 4 x 4 outputs per thread and loads one
 // shared-memory value per FMA, which holds FP32 near 30% of the pipe. Here
 // each thread reads two float4 of A and two of B per k (an 8 x 8 outer

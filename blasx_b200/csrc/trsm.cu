@@ -72,8 +72,8 @@ template <typename T> __device__ __forceinline__ void copy_or_zero(T *dst, const
 // B). Each vector is scaled by `scale` (alpha) on load.
 //
 // What bounds it: the chain of bs dependent steps of each vector (a
-// reciprocal multiply, a shuffle and a multiply-add, ~60 cycles), and beside
-// it the FP64 pipe. So a block is as tall as its vectors fit in registers, one
+// reciprocal multiply, a shuffle and a multiply-add; about 210 cycles a step
+// with the barrier and the copies of its panel), and beside it the FP64 pipe. So a block is as tall as its vectors fit in registers, one
 // launch instead of four substitutions of 64 rows with three updates between
 // them; every warp runs its own vectors, the rows after step k updated by all
 // lanes at once, and a step needs no barrier. S passes through shared memory
