@@ -74,6 +74,36 @@ def test_unmatched_scales_keep_the_bound(blx, dt, shape, kind, ta, tb):
     check(out, A, B, C, 1.5, -0.5, k, dt)
 
 
+@pytest.mark.parametrize("dt,shape", [("d", (2100, 1900, 512)), ("s", (1024, 1024, 300))])
+def test_few_entries_that_meet_keep_the_bound(blx, dt, shape):
+    # one entry in ten: a row and a column share a few dozen products or fewer
+    m, n, k = shape
+    A, B, C = operands(dt, m, n, k, "even")
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(5)
+    A, B = (x * (torch.rand(x.shape, device="cuda", generator=gen) < 0.1) for x in (A, B))
+    out = C.clone()
+    rc = blx.gemm_device("N", "N", m, n, k, 1.0, A, m, B, k, 0.0, out, m, dtype=dt)
+    assert rc == blx.BLASX_OK, blx.last_error()
+    torch.cuda.synchronize()
+    check(out, A, B, C, 1.0, 0.0, k, dt)
+
+
+@pytest.mark.parametrize("dt,shape", [("d", (1300, 1300, 1300)), ("d", (2100, 1900, 1600)), ("z", (900, 900, 900))])
+def test_decaying_kernels_keep_the_bound(blx, dt, shape):
+    # entries that fall off from the diagonal: far from C's diagonal every product is tiny
+    m, n, k = shape
+    at = [torch.arange(x, device="cuda", dtype=torch.float64) / x for x in (m, n, k)]
+    A = torch.exp(-((at[2][:, None] - at[0][None, :]) / 0.1) ** 2).to(T[dt])
+    B = torch.exp(-((at[2][None, :] - at[1][:, None]) / 0.1) ** 2).to(T[dt])
+    C = torch.zeros((n, m), dtype=T[dt], device="cuda")
+    out = C.clone()
+    rc = blx.gemm_device("N", "N", m, n, k, 1.0, A.contiguous(), m, B.contiguous(), k, 0.0, out, m, dtype=dt)
+    assert rc == blx.BLASX_OK, blx.last_error()
+    torch.cuda.synchronize()
+    check(out, A, B, C, 1.0, 0.0, k, dt)
+
+
 @pytest.mark.parametrize("dt,shape", SIZES)
 def test_matched_scales_stay_emulated(blx, dt, shape):
     # large meets large: nothing is lost, and the call keeps its path
